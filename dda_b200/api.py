@@ -77,6 +77,7 @@ def lib():
         "dda_cancel": ([vp], ctypes.c_int),
         "dda_launch_count": ([vp], ctypes.c_int64),
         "dda_matvec_layout": ([vp, ctypes.POINTER(ctypes.c_int64)], ctypes.c_int),
+        "dda_matvec_passes": ([vp], ctypes.c_int),
         "dda_profile_matvec": ([vp, ctypes.c_int, ctypes.c_int, dp], ctypes.c_int),
         "dda_synchronize": ([vp], ctypes.c_int),
         "dda_far_field": ([vp, ctypes.c_int, dp, ctypes.c_int64, dp, dp], ctypes.c_int),
@@ -504,11 +505,17 @@ class CudaMatVec:
         keys = ("yz_path", "clusters", "cluster_size", "rows_per_batch", "smem_yz", "lines_per_x_tile",
                 "compile_time_plans", "device_bytes")
         d = dict(zip(keys, (int(x) for x in v)))
-        d["yz_path"] = ("fused", "cluster", "split")[d["yz_path"]]
+        d["yz_path"] = ("fused", "cluster", "split", "passes")[d["yz_path"]]
         if d["yz_path"] == "fused":  # slots 1, 2: CTAs per plane and thread groups
             d["groups"] = d.pop("cluster_size")
             d["ctas_per_plane"] = d.pop("clusters")
         return d
+
+    @property
+    def passes(self):
+        """True when matvecs run their y/z passes as three kernels over a work
+        buffer instead of the plane kernel that `layout` describes."""
+        return bool(lib().dda_matvec_passes(self.h))
 
     def profile(self, nrhs=1, reps=10):
         """Mean ms of the matvec stages: x forward, y/z, x inverse, total."""

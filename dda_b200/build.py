@@ -13,11 +13,14 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libdda_b200.so")
 SOURCES = ["dda_cuda.cu", "frontend.cpp", "serve.cpp"]
-# mv_inst.cu is compiled once per (part, double): the kernel-table parts
-MV_PARTS = [(part, dbl) for dbl in (0, 1) for part in (0, 1, 2, 3, 4, 5)]
+# mv_inst.cu is compiled once per (part, double, sub): the kernel-table parts,
+# those with a kernel per grid length once per range of lengths
+MV_PARTS = [(part, dbl, sub) for dbl in (0, 1) for part in (6, 0, 5, 2, 4, 3, 1)
+            for sub in (range(4) if part in (0, 5, 6) else (0,))]
 HEADERS = ["fft_engine.cuh", "fft_plan.cuh", "reduce.cuh", "krylov_ops.cuh", "krylov_kernels.cuh",
            "matvec_kernels.cuh", "matvec_planned.cuh", "matvec_dispatch.cuh", "dmatrix_kernels.cuh",
-           "farfield_kernels.cuh", "matvec_slot.cuh", "kernel_shapes.cuh", "matvec_pair.cuh"]
+           "farfield_kernels.cuh", "matvec_slot.cuh", "kernel_shapes.cuh", "matvec_pair.cuh",
+           "matvec_pass.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -49,9 +52,9 @@ def _units():
     units = []
     for f in SOURCES:
         units.append((os.path.join(CSRC, f), os.path.join(OBJ, f + ".o"), []))
-    for part, dbl in MV_PARTS:
-        units.append((os.path.join(CSRC, "mv_inst.cu"), os.path.join(OBJ, "mv_inst_%d_%d.o" % (part, dbl)),
-                      ["-DDDA_MV_PART=%d" % part, "-DDDA_MV_DOUBLE=%d" % dbl]))
+    for part, dbl, sub in MV_PARTS:
+        units.append((os.path.join(CSRC, "mv_inst.cu"), os.path.join(OBJ, "mv_inst_%d_%d_%d.o" % (part, dbl, sub)),
+                      ["-DDDA_MV_PART=%d" % part, "-DDDA_MV_DOUBLE=%d" % dbl, "-DDDA_MV_SUB=%d" % sub]))
     return units
 
 

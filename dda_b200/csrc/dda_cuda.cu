@@ -109,6 +109,8 @@ struct FftPlan {
   std::vector<int> pos_h;  // frequency -> position after a forward transform
   float2* tw32 = nullptr;
   double2* tw64 = nullptr;
+  float2* stw32 = nullptr;   // compile-time plans: stage twiddles, butterfly-major (StageTw)
+  double2* stw64 = nullptr;
   int* freq = nullptr;     // device: position -> frequency
   int* pos = nullptr;      // device: frequency -> position
 
@@ -143,6 +145,23 @@ struct FftPlan {
     dmalloc((void**)&tw32, n * sizeof(float2));
     CK(cudaMemcpyAsync(tw64, h64.data(), n * sizeof(double2), cudaMemcpyHostToDevice, g_alloc_stream));
     CK(cudaMemcpyAsync(tw32, h32.data(), n * sizeof(float2), cudaMemcpyHostToDevice, g_alloc_stream));
+    std::vector<double2> s64;
+    std::vector<float2> s32;
+    if (!radices.empty()) {
+      for (int i = 0, L = n; i < (int)radix.size() && L > radix[i]; L /= radix[i], i++)
+        for (int m = 1; m < radix[i]; m++)
+          for (int j = 0; j < L / radix[i]; j++) {
+            s64.push_back(h64[(size_t)j * m * (n / L)]);
+            const float2 w = h32[(size_t)j * m * (n / L)];
+            s32.push_back(w);
+          }
+      s64.push_back(make_double2(0, 0));  // the kernels copy an even count
+      s32.push_back(make_float2(0, 0));
+      dmalloc((void**)&stw64, s64.size() * sizeof(double2));
+      dmalloc((void**)&stw32, s32.size() * sizeof(float2));
+      CK(cudaMemcpyAsync(stw64, s64.data(), s64.size() * sizeof(double2), cudaMemcpyHostToDevice, g_alloc_stream));
+      CK(cudaMemcpyAsync(stw32, s32.data(), s32.size() * sizeof(float2), cudaMemcpyHostToDevice, g_alloc_stream));
+    }
     // Mixed-radix digit reversal of the decimation-in-frequency transform:
     // frequency k = d0 + R0 d1 + R0 R1 d2 + ... sits at position
     // d0 n/R0 + d1 n/(R0 R1) + ...
@@ -174,7 +193,15 @@ struct FftPlan {
     d.freq = freq;
     return d;
   }
+  template <typename TW> const TW* stage_tw() const {
+    if constexpr (std::is_same<TW, float2>::value) return stw32;
+    else return stw64;
+  }
   void release(cudaStream_t s) {
+    if (stw32) cudaFreeAsync(stw32, s);
+    if (stw64) cudaFreeAsync(stw64, s);
+    stw32 = nullptr;
+    stw64 = nullptr;
     if (tw32) cudaFreeAsync(tw32, s);
     if (tw64) cudaFreeAsync(tw64, s);
     if (freq) cudaFreeAsync(freq, s);
@@ -203,6 +230,9 @@ template <typename T> struct Engine {
   T2* ccs = nullptr;   // [max_rhs][nmat][3] scaled sqrt(cc)
   T2* xhat = nullptr;  // [max_rhs][Gx][3][nlines]
   T2* zbuf = nullptr;  // split path [max_rhs][Gx][3][Gz][by]
+  void* pbuf = nullptr;       // work buffer of the y/z passes (matvec_pass.cuh)
+  size_t pbuf_bytes = 0;
+  bool pass = false;          // the y/z passes exist for this grid
   T2* vec[10] = {};    // Krylov vectors [max_rhs][3 nvs]
   T2* io = nullptr;    // host-API staging [max_rhs][3 nvs]
   T2* xo = nullptr;    // MIXED, FP64 engine: refined solution x and b = sqrt(cc) Einc
@@ -225,11 +255,12 @@ template <typename T> struct Engine {
   MvKernels<T> k;
   void release(cudaStream_t s) {
     for (void* p : {(void*)dc, (void*)ccs, (void*)xhat, (void*)zbuf, (void*)io, (void*)slots, (void*)order,
-                    (void*)xo, (void*)bo})
+                    (void*)xo, (void*)bo, pbuf})
       if (p) cudaFreeAsync(p, s);
     for (auto& v : vec)
       if (v) cudaFreeAsync(v, s);
     dc = ccs = xhat = zbuf = io = slots = xo = bo = nullptr;
+    pbuf = nullptr;
     order = nullptr;
     for (auto& v : vec) v = nullptr;
   }
@@ -405,7 +436,7 @@ template <typename T> void setup_slot(dda_ctx* c, Engine<T>& e) {
   }
   e.order = (uint32_t*)dalloc<float>(order.size() * sizeof(uint32_t));
   CK(cudaMemcpyAsync(e.order, order.data(), order.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
-  e.slots = (T2*)dalloc<T>((size_t)ncl_max * g.Gz * sg.wp * sizeof(T2));
+  if (!e.pass) e.slots = (T2*)dalloc<T>((size_t)ncl_max * g.Gz * sg.wp * sizeof(T2));
   e.sg = sg;
   e.cl = cl;
   e.ncl = ncl;
@@ -477,6 +508,36 @@ template <typename T> void pick_x_tile(dda_ctx* c, Engine<T>& e) {
   e.smem_x = ((size_t)g.Gx + g.nmat + (size_t)e.tl * g.pitchx) * s;
 }
 
+// Whether a grid's y/z passes run as the three kernels of matvec_pass.cuh.
+// Against the plane kernels (whole matvec, FP32, one / two right-hand sides,
+// kernels replayed from a graph): 56^3 24.8 -> 21.3 / 25.2 -> 23.8 us, 80^3
+// 34.7 -> 29.1 / 57.2 -> 36.8, 128^3 79.8 -> 54.9 / 148 -> 91, 200^3 472 -> 214
+// / 876 -> 420; FP64 80^3 55.3 -> 39.2 / 97.6 -> 58.0.  Against the
+// runtime-planned plane kernel, from 10^3 (22.2 -> 14.1) to 50^3 (52.1 ->
+// 20.3).  Up to 48 x 48 planes the planned plane kernel is one launch of 5 to
+// 9 us, and two launches more cost what the passes gain: 32^3 15.0 -> 17.5 us
+// replayed, 48^3 20.7 -> 19.5 replayed but 11.7 -> 13.4 launched one by one.
+inline bool pass_grid(long long Gx, long long Gy, long long Gz, uint32_t flags) {
+  if (flags & (DDA_FLAG_SPLIT_YZ | DDA_FLAG_SLOT_YZ | DDA_FLAG_RUNTIME_PLANS | DDA_FLAG_YZ_GROUPS2 |
+               DDA_FLAG_YZ_GROUPS4 | DDA_FLAG_YZ_PAIR))
+    return false;
+  if (!has_plan((int)Gx) || !has_plan((int)Gy) || !has_plan((int)Gz)) return false;
+  return !(has_tuned_plan((int)Gx) && Gy == Gz && (Gy == 32 || Gy == 48));
+}
+
+// Work buffer of the y/z passes: all planes of all right-hand sides, or as
+// much of them as kPassCap holds, and at least the two planes of a frequency
+// for one pair.  y/z passes of the 128-rhs spheroid (4.8 GB in all) with
+// buffers of 64 MB, 256 MB, 1 GB and all: 6.53, 5.72, 5.39, 5.32 ms -- each
+// chunk is three launches with a tail, and staying in L2 does not make up for
+// them; 512^3 (two right-hand sides, 3.2 GB) 6.73, 6.15, 5.93, 5.84 ms.
+constexpr size_t kPassCap = (size_t)1 << 30;
+inline size_t pass_buffer_bytes(long long Gx, long long Gz, long long by, int max_rhs, size_t s) {
+  const size_t plane = (size_t)(Gz * 3 * by) * s;
+  const size_t all = (size_t)(max_rhs + 1) / 2 * 2 * (2 * (Gx / 2 + 1)) * plane;
+  return std::max(4 * plane, std::min(all, kPassCap));
+}
+
 // Chooses tile shapes and allocates the matvec buffers of one precision.
 template <typename T> void setup_engine(dda_ctx* c) {
   typedef typename C2<T>::t T2;
@@ -528,8 +589,9 @@ template <typename T> void setup_engine(dda_ctx* c) {
     e.yz.nrw = nrw - nrw % forced;  // a multiple of the groups: an equal share each
     e.smem_yz = fixed + e.yz.nrw * row;
   }
+  e.pass = pass_grid(g.Gx, g.Gy, g.Gz, c->flags);
   if (!e.fused && e.k.slot && !(c->flags & DDA_FLAG_SPLIT_YZ)) setup_slot<T>(c, e);
-  if (!e.fused && !e.slot_path) {
+  if (!e.fused && !e.slot_path && !e.pass) {
     // split path: zbuf, k_yrows over NW rows per CTA, column FFTs along z
     e.yz.nrw = NW;
     e.smem_rows = ((size_t)g.Gy + (size_t)NW * 3 * y.py) * s;
@@ -562,20 +624,35 @@ template <typename T> void setup_engine(dda_ctx* c) {
   }
   pick_x_tile<T>(c, e);
   if (e.smem_x > kSmemMax) throw DdaError(DDA_ERR_UNSUPPORTED, "grid x extent too large");
+  // (a kernel that stays within the 48 KB every kernel may use is not looked
+  // up here: that would load it, with all others of its context, at creation)
   auto attr = [](const void* f, size_t bytes) {
+    if (bytes <= 48 * 1024) return;
     if (bytes > kSmemMax) throw DdaError(DDA_ERR_UNSUPPORTED, "shared-memory tile above the SM limit");
     CK(allow_smem(f));
   };
   for (const void* f : x_pass_kernels(e)) attr(f, e.smem_x);
-  if (e.fused) {
+  if (e.fused && !e.pass) {  // the autotuner may take up to all of it
     for (int gr : {1, 2, 4})
-      if (fused_yz<T>(e, gr)) attr((const void*)fused_yz<T>(e, gr), e.smem_yz);
+      if (fused_yz<T>(e, gr)) attr((const void*)fused_yz<T>(e, gr), kSmemMax);
     for (auto f : e.k.pair)
-      if (f) attr((const void*)f, e.smem_yz);
+      if (f) attr((const void*)f, kSmemMax);
   }
-  else if (!e.slot_path) {
+  else if (!e.slot_path && !e.pass) {
     attr((const void*)e.k.yrows, e.smem_rows);
     attr((const void*)e.k.cols, e.smem_cols);
+  }
+  if (e.pass) {
+    auto attrs = [&](const auto& k) {
+      if (!k.rows) return;
+      attr((const void*)k.zfwd, k.smem_z);
+      attr((const void*)k.zinv, k.smem_z);
+      attr((const void*)k.rows, k.smem_rows);
+    };
+    attrs(e.k.pass1);
+    if (c->max_rhs > 1) attrs(e.k.pass2);
+    e.pbuf_bytes = pass_buffer_bytes(g.Gx, g.Gz, g.by, c->max_rhs, s);
+    e.pbuf = dalloc<T>(e.pbuf_bytes);
   }
   const int hx = g.Gx / 2 + 1, hy = g.Gy / 2 + 1, hz = g.Gz / 2 + 1;
   e.dc = (T2*)dalloc<T>((size_t)hx * hy * hz * 6 * s);
@@ -621,13 +698,53 @@ RedTarget red_target(dda_ctx* c, int nparts) {
   return t;
 }
 
-// The y/z passes: the fused plane kernel, the cluster kernel, or the split
-// path (column FFTs along z around the row kernel).
+// The y/z passes through the work buffer, W right-hand sides at a time.
+template <typename T, int W>
+int launch_pass(dda_ctx* c, const PassKernels<T, W>& k, int nrhs, cudaStream_t s, KrylovState* st, int skipmv) {
+  typedef typename PassV<T, W>::t V;
+  Engine<T>& e = eng<T>(c);
+  const MvGeom& g = c->g;
+  const int E = (nrhs + W - 1) / W, hx = g.Gx / 2 + 1, w3 = 3 * g.by;
+  const size_t pair = 2 * (size_t)g.Gz * w3 * sizeof(V);
+  const int fit = (int)std::max<size_t>(1, std::min<size_t>(e.pbuf_bytes / pair, (size_t)E * hx));
+  const int ec = std::min(E, fit), axc = std::max(1, fit / ec);
+  PassGeom p;
+  p.Gx = g.Gx; p.Gy = g.Gy; p.Gz = g.Gz;
+  p.by = g.by; p.bz = g.bz; p.nb = g.by * g.bz;
+  p.nrhs = nrhs;
+  p.xpos = c->mx.pos;
+  V* buf = (V*)e.pbuf;
+  const int ztiles = (w3 + k.ztc - 1) / k.ztc;
+  int launches = 0;
+  for (int e0 = 0; e0 < E; e0 += ec)
+    for (int ax = 0; ax < hx; ax += axc) {
+      p.b0 = e0 * W;
+      p.ax0 = ax;
+      p.nax = std::min(axc, hx - ax);
+      const int ne = std::min(ec, E - e0);
+      const dim3 gz(ztiles, 2 * p.nax, ne);
+      k.zfwd<<<gz, k.ntf, k.smem_z, s>>>(e.xhat, buf, p, c->mz.stage_tw<typename C2<T>::t>(), st, skipmv);
+      k.rows<<<dim3((g.Gz / 2 + 1) * k.rows_per, p.nax, ne), k.ntr, k.smem_rows, s>>>(
+          buf, e.dc, p, c->my.stage_tw<typename C2<T>::t>(), st, skipmv);
+      k.zinv<<<gz, k.nti, k.smem_z, s>>>(e.xhat, buf, p, c->mz.stage_tw<typename C2<T>::t>(), st, skipmv);
+      launches += 3;
+    }
+  return launches;
+}
+
+// The y/z passes: the kernels of matvec_pass.cuh, or the fused plane kernel,
+// the cluster kernel or the split path (column FFTs along z around the row
+// kernel).  Returns the number of launches.
 template <typename T>
-void launch_yz(dda_ctx* c, int nrhs, cudaStream_t s, KrylovState* st, int skipmv) {
+int launch_yz(dda_ctx* c, int nrhs, cudaStream_t s, KrylovState* st, int skipmv) {
   Engine<T>& e = eng<T>(c);
   const MvGeom& g = c->g;
   const FftPlanDev py = c->my.dev<T>(), pz = c->mz.dev<T>();
+  if (e.pass) {
+    if constexpr (sizeof(T) == 4)
+      if (nrhs > 1) return launch_pass<T, 2>(c, e.k.pass2, nrhs, s, st, skipmv);
+    return launch_pass<T, 1>(c, e.k.pass1, nrhs, s, st, skipmv);
+  }
   if (e.fused && e.yz_pair) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
@@ -669,7 +786,9 @@ void launch_yz(dda_ctx* c, int nrhs, cudaStream_t s, KrylovState* st, int skipmv
     dim3 gr((g.Gz + e.yz.nrw - 1) / e.yz.nrw, g.Gx, nrhs);
     e.k.yrows<<<gr, kNtYz, e.smem_rows, s>>>(e.zbuf, e.dc, g, e.yz, py, st, skipmv);
     e.k.cols<<<gc, kNtC, e.smem_cols, s>>>(e.zbuf, e.xhat, e.cz_inv, pz, 1, st, skipmv);
+    return 3;
   }
+  return 1;
 }
 
 // ------------------------------------------------------------ autotune ----
@@ -724,7 +843,7 @@ template <typename T> void apply_choice(dda_ctx* c, Engine<T>& e, const TuneChoi
 template <typename T> void autotune(dda_ctx* c) {
   Engine<T>& e = eng<T>(c);
   const MvGeom& g = c->g;
-  if (!e.on || !(e.fused || e.slot_path)) return;
+  if (!e.on || e.pass || !(e.fused || e.slot_path)) return;
   NvtxRange range(sizeof(T) == 4 ? "dda autotune fp32" : "dda autotune fp64");
   if ((long long)g.Gx * g.Gy * g.Gz < (1LL << 20)) return;  // small grids keep the defaults
   // the box changes the best batching little next to the grid, so shapes
@@ -830,11 +949,11 @@ void matvec(dda_ctx* c, const A2* arg, A2* res, int conj, int nrhs, cudaStream_t
     pre.step.red = red;
   }
   xf<<<gx, kNtX, e.smem_x, s>>>(arg, e.xhat, c->line_off, c->dip, c->perm, e.ccs, conj, g, px, st, skipmv, pre);
-  launch_yz<T>(c, nrhs, s, st, skipmv);
+  const int n = launch_yz<T>(c, nrhs, s, st, skipmv);
   step.red = red;
   xi<<<gx, kNtX, e.smem_x, s>>>(arg, res, e.xhat, c->line_off, c->dip, c->perm, e.ccs, conj, g, px, st, step, skipmv);
   CK(cudaGetLastError());
-  c->launches += (e.fused || e.slot_path) ? 3 : 5;
+  c->launches += 2 + n;
 }
 
 // D-matrix generation (FP64) into the enabled engines' octants.
@@ -1572,11 +1691,12 @@ int dda_create(const dda_problem* p, int precision, dda_ctx** out) {
     c->px.create(g.Gx);
     c->py.create(g.Gy);
     c->pz.create(g.Gz);
-    c->planned = has_tuned_plan(g.Gx) && has_tuned_plan(g.Gy) && has_tuned_plan(g.Gz) &&
-                 !(c->flags & DDA_FLAG_RUNTIME_PLANS);
-    c->mx.create(g.Gx, c->planned ? tuned_radices(g.Gx) : std::vector<int>());
-    c->my.create(g.Gy, c->planned ? tuned_radices(g.Gy) : std::vector<int>());
-    c->mz.create(g.Gz, c->planned ? tuned_radices(g.Gz) : std::vector<int>());
+    c->planned = pass_grid(g.Gx, g.Gy, g.Gz, c->flags) ||
+                 (has_tuned_plan(g.Gx) && has_tuned_plan(g.Gy) && has_tuned_plan(g.Gz) &&
+                  !(c->flags & DDA_FLAG_RUNTIME_PLANS));
+    c->mx.create(g.Gx, c->planned ? plan_radices(g.Gx) : std::vector<int>());
+    c->my.create(g.Gy, c->planned ? plan_radices(g.Gy) : std::vector<int>());
+    c->mz.create(g.Gz, c->planned ? plan_radices(g.Gz) : std::vector<int>());
     g.fx = c->mx.freq;
     g.fy = c->my.freq;
     g.fz = c->mz.freq;
@@ -2095,6 +2215,7 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
                        !(p->flags & DDA_FLAG_RUNTIME_PLANS);
   long long bytes = 4 * (nl + 1) + 9 * nv;                    // line offsets, dipoles, permutation, materials
   bytes += 6 * (Gx + Gy + Gz) * (8 + 16 + 4 + 4);              // plans
+  bytes += 4 * (Gx + Gy + Gz) * (8 + 16);                      // their stage twiddles
   auto engine = [&](long long s) {
     long long e = (Gx / 2 + 1) * (Gy / 2 + 1) * (Gz / 2 + 1) * 6 * s;  // D-hat octant
     // vectors: 10 Krylov + io; MIXED keeps two more in FP64 (x, b) and only
@@ -2108,7 +2229,9 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
     DDA_FUSED_LENGTHS(C)
 #undef C
     const bool has_yz = !planned || (Gy == Gz && fused_len);
-    if (!(has_yz && smem_yz <= (long long)kSmemMax) || (p->flags & (DDA_FLAG_SPLIT_YZ | DDA_FLAG_SLOT_YZ)))
+    if (pass_grid(Gx, Gy, Gz, p->flags))
+      e += (long long)pass_buffer_bytes(Gx, Gz, by, (int)R, (size_t)s);
+    else if (!(has_yz && smem_yz <= (long long)kSmemMax) || (p->flags & (DDA_FLAG_SPLIT_YZ | DDA_FLAG_SLOT_YZ)))
       e += R * Gx * 3 * Gz * by * s;
     return e;
   };
@@ -2129,11 +2252,11 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
 int dda_matvec_layout(const dda_ctx* ctx, int64_t* out) {
   if (!ctx || !out) return DDA_ERR_ARG;
   auto fill = [&](const auto& e) {
-    out[0] = e.fused ? 0 : e.slot_path ? 1 : 2;
+    out[0] = e.fused ? 0 : e.slot_path ? 1 : e.pass ? 3 : 2;
     out[1] = e.fused ? (e.yz_pair ? 2 : 1) : e.ncl;
     out[2] = e.fused ? e.yz_groups : e.cl;
     out[3] = e.slot_path ? e.sg.nrw : e.yz.nrw;
-    out[4] = (int64_t)(e.fused ? e.smem_yz : e.slot_path ? e.smem_slot : e.smem_rows);
+    out[4] = (int64_t)(e.fused ? e.smem_yz : e.slot_path ? e.smem_slot : e.pass ? e.k.pass1.smem_rows : e.smem_rows);
   };
   if (ctx->e32.on) fill(ctx->e32);
   else fill(ctx->e64);
@@ -2141,6 +2264,11 @@ int dda_matvec_layout(const dda_ctx* ctx, int64_t* out) {
   out[6] = ctx->planned ? 1 : 0;
   out[7] = (int64_t)ctx->dev_bytes;
   return DDA_OK;
+}
+
+int dda_matvec_passes(const dda_ctx* ctx) {
+  if (!ctx) return 0;
+  return (ctx->e32.on ? ctx->e32.pass : ctx->e64.pass) ? 1 : 0;
 }
 
 int dda_profile_matvec(dda_ctx* ctx, int nrhs, int reps, double* ms) {

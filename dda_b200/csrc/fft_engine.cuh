@@ -37,33 +37,118 @@ template <typename T> struct C2;
 template <> struct C2<float> { typedef float2 t; };
 template <> struct C2<double> { typedef double2 t; };
 
+__host__ __device__ __forceinline__ float2 f2add(float2 a, float2 b) {
+#ifdef DDA_F32X2
+  return __fadd2_rn(a, b);
+#else
+  return make_float2(a.x + b.x, a.y + b.y);
+#endif
+}
+__host__ __device__ __forceinline__ float2 f2mul(float2 a, float2 b) {
+#ifdef DDA_F32X2
+  return __fmul2_rn(a, b);
+#else
+  return make_float2(a.x * b.x, a.y * b.y);
+#endif
+}
+__host__ __device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) {
+#ifdef DDA_F32X2
+  return __ffma2_rn(a, b, c);
+#else
+  return make_float2(a.x * b.x + c.x, a.y * b.y + c.y);
+#endif
+}
+
+// Two complex64 values side by side (two right-hand sides), real parts and
+// imaginary parts packed: every operation on them is one two-lane
+// instruction, and each lane is rounded as the same operation on one value.
+struct __align__(16) P2 {
+  float2 r, i;
+};
+// Real type of a complex value type, and the type of its twiddles.
+template <typename V> struct CxTraits;
+template <> struct CxTraits<float2> { typedef float T; typedef float2 W; };
+template <> struct CxTraits<double2> { typedef double T; typedef double2 W; };
+template <> struct CxTraits<P2> { typedef float T; typedef float2 W; };
+
 template <typename T2> __host__ __device__ __forceinline__ T2 czero() {
   T2 r; r.x = 0; r.y = 0; return r;
 }
-template <typename T2> __host__ __device__ __forceinline__ T2 cmul(T2 a, T2 b) {
-  T2 r;
+template <> __host__ __device__ __forceinline__ P2 czero<P2>() {
+  P2 r; r.r = make_float2(0, 0); r.i = make_float2(0, 0); return r;
+}
+// Products and fused products are written out operation by operation: what
+// the compiler would contract could differ from one kernel to the next, and a
+// right-hand side has the same bits alone, in a batch and on every path.
+__host__ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
+  float2 r;
+#ifdef __CUDA_ARCH__
+  r.x = __fmaf_rn(-a.y, b.y, __fmul_rn(a.x, b.x));
+  r.y = __fmaf_rn(a.y, b.x, __fmul_rn(a.x, b.y));
+#else
   r.x = a.x * b.x - a.y * b.y;
   r.y = a.x * b.y + a.y * b.x;
+#endif
+  return r;
+}
+__host__ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+  double2 r;
+#ifdef __CUDA_ARCH__
+  r.x = __fma_rn(-a.y, b.y, __dmul_rn(a.x, b.x));
+  r.y = __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y));
+#else
+  r.x = a.x * b.x - a.y * b.y;
+  r.y = a.x * b.y + a.y * b.x;
+#endif
   return r;
 }
 template <typename T2> __host__ __device__ __forceinline__ T2 cadd(T2 a, T2 b) {
-#ifdef DDA_F32X2
-  if constexpr (std::is_same<T2, float2>::value) return __fadd2_rn(a, b);
-#endif
+  if constexpr (std::is_same<T2, float2>::value) return f2add(a, b);
   T2 r; r.x = a.x + b.x; r.y = a.y + b.y; return r;
 }
 template <typename T2> __host__ __device__ __forceinline__ T2 csub(T2 a, T2 b) {
-#ifdef DDA_F32X2
-  if constexpr (std::is_same<T2, float2>::value) return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);  // exact -b
-#endif
+  if constexpr (std::is_same<T2, float2>::value) return f2fma(b, make_float2(-1.0f, -1.0f), a);  // exact -b
   T2 r; r.x = a.x - b.x; r.y = a.y - b.y; return r;
 }
 // acc + c t for a real c
 template <typename T, typename T2> __host__ __device__ __forceinline__ T2 caxr(T2 acc, T c, T2 t) {
-#ifdef DDA_F32X2
-  if constexpr (std::is_same<T2, float2>::value) return __ffma2_rn(make_float2(c, c), t, acc);
-#endif
-  acc.x += c * t.x; acc.y += c * t.y; return acc;
+  if constexpr (std::is_same<T2, float2>::value) return f2fma(make_float2(c, c), t, acc);
+  acc.x = fma(c, t.x, acc.x); acc.y = fma(c, t.y, acc.y); return acc;
+}
+// acc + d v for a complex d: two fused steps per part
+__device__ __forceinline__ float2 cfma(float2 acc, float2 d, float2 v) {
+  acc.x = __fmaf_rn(-d.y, v.y, __fmaf_rn(d.x, v.x, acc.x));
+  acc.y = __fmaf_rn(d.y, v.x, __fmaf_rn(d.x, v.y, acc.y));
+  return acc;
+}
+__device__ __forceinline__ double2 cfma(double2 acc, double2 d, double2 v) {
+  acc.x = __fma_rn(-d.y, v.y, __fma_rn(d.x, v.x, acc.x));
+  acc.y = __fma_rn(d.y, v.x, __fma_rn(d.x, v.y, acc.y));
+  return acc;
+}
+__host__ __device__ __forceinline__ P2 cmul(P2 a, float2 w) {
+  const float2 wx = make_float2(w.x, w.x), wy = make_float2(w.y, w.y), ny = make_float2(-w.y, -w.y);
+  P2 r;
+  r.r = f2fma(a.i, ny, f2mul(a.r, wx));
+  r.i = f2fma(a.i, wx, f2mul(a.r, wy));
+  return r;
+}
+template <> __host__ __device__ __forceinline__ P2 cadd<P2>(P2 a, P2 b) {
+  P2 r; r.r = f2add(a.r, b.r); r.i = f2add(a.i, b.i); return r;
+}
+template <> __host__ __device__ __forceinline__ P2 csub<P2>(P2 a, P2 b) {
+  const float2 m = make_float2(-1.0f, -1.0f);
+  P2 r; r.r = f2fma(b.r, m, a.r); r.i = f2fma(b.i, m, a.i); return r;
+}
+template <> __host__ __device__ __forceinline__ P2 caxr<float, P2>(P2 acc, float c, P2 t) {
+  const float2 cc = make_float2(c, c);
+  acc.r = f2fma(cc, t.r, acc.r); acc.i = f2fma(cc, t.i, acc.i); return acc;
+}
+__device__ __forceinline__ P2 cfma(P2 acc, float2 d, P2 v) {
+  const float2 dx = make_float2(d.x, d.x), dy = make_float2(d.y, d.y), ny = make_float2(-d.y, -d.y);
+  acc.r = f2fma(ny, v.i, f2fma(dx, v.r, acc.r));
+  acc.i = f2fma(dy, v.r, f2fma(dx, v.i, acc.i));
+  return acc;
 }
 // a complex value in another precision (round to nearest)
 template <typename T2, typename S2> __host__ __device__ __forceinline__ T2 cvt(S2 a) {
@@ -75,8 +160,38 @@ template <typename T2> __host__ __device__ __forceinline__ T2 cconj(T2 a) {
 // multiply by -i (forward) or +i (inverse)
 template <bool INV, typename T2> __host__ __device__ __forceinline__ T2 mul_mi(T2 a) {
   T2 r;
-  if (INV) { r.x = -a.y; r.y = a.x; } else { r.x = a.y; r.y = -a.x; }
+  if constexpr (std::is_same<T2, P2>::value) {
+    if (INV) { r.r = make_float2(-a.i.x, -a.i.y); r.i = a.r; }
+    else { r.r = a.i; r.i = make_float2(-a.r.x, -a.r.y); }
+  } else {
+    if (INV) { r.x = -a.y; r.y = a.x; } else { r.x = a.y; r.y = -a.x; }
+  }
   return r;
+}
+// a + mul_mi<INV>(b) and a - mul_mi<INV>(b): the exchange of b's parts and
+// their signs go into the additions.
+template <bool INV, typename T2> __host__ __device__ __forceinline__ T2 cadd_mi(T2 a, T2 b) {
+  if constexpr (std::is_same<T2, P2>::value) {
+    const float2 m = make_float2(-1.0f, -1.0f);
+    P2 r;
+    if (INV) { r.r = f2fma(b.i, m, a.r); r.i = f2add(a.i, b.r); }
+    else { r.r = f2add(a.r, b.i); r.i = f2fma(b.r, m, a.i); }
+    return r;
+  } else {
+    if (INV) { a.x -= b.y; a.y += b.x; } else { a.x += b.y; a.y -= b.x; }
+  }
+  return a;
+}
+template <bool INV, typename T2> __host__ __device__ __forceinline__ T2 csub_mi(T2 a, T2 b) {
+  return cadd_mi<!INV>(a, b);
+}
+template <typename T2> __host__ __device__ __forceinline__ T2 cneg(T2 a) {
+  if constexpr (std::is_same<T2, P2>::value) {
+    a.r = make_float2(-a.r.x, -a.r.y); a.i = make_float2(-a.i.x, -a.i.y);
+  } else {
+    a.x = -a.x; a.y = -a.y;
+  }
+  return a;
 }
 
 constexpr int kMaxStages = 16;
@@ -91,46 +206,68 @@ struct FftPlanDev {
 };
 
 // ------------------------------------------------------------ DFT cores ----
-template <int R, bool INV, typename T2> struct Dft;
+// DFT of R values in registers.  NZ: inputs v[NZ..R) are zero padding (their
+// registers are not read), so the additions of them fold away; the result is
+// that of the full DFT.
+template <int R, bool INV, typename T2, int NZ = R> struct Dft;
 
-template <bool INV, typename T2> struct Dft<2, INV, T2> {
+template <bool INV, typename T2, int NZ> struct Dft<2, INV, T2, NZ> {
   static __host__ __device__ __forceinline__ void run(T2* v) {
-    T2 a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
+    if constexpr (NZ == 1) {
+      v[1] = v[0];
+    } else {
+      T2 a = v[0], b = v[1];
+      v[0] = cadd(a, b);
+      v[1] = csub(a, b);
+    }
   }
 };
 
-template <bool INV, typename T2> struct Dft<4, INV, T2> {
+template <bool INV, typename T2, int NZ> struct Dft<4, INV, T2, NZ> {
   static __host__ __device__ __forceinline__ void run(T2* v) {
-    T2 t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]);
-    T2 t2 = cadd(v[1], v[3]), t3 = mul_mi<INV>(csub(v[1], v[3]));
-    v[0] = cadd(t0, t2);
-    v[2] = csub(t0, t2);
-    v[1] = cadd(t1, t3);
-    v[3] = csub(t1, t3);
+    if constexpr (NZ == 1) {
+      v[1] = v[2] = v[3] = v[0];
+    } else {
+      T2 t0 = v[0], t1 = v[0], t2 = v[1], t3 = v[1];
+      if constexpr (NZ > 2) { t0 = cadd(v[0], v[2]); t1 = csub(v[0], v[2]); }
+      if constexpr (NZ > 3) { t2 = cadd(v[1], v[3]); t3 = csub(v[1], v[3]); }
+      v[0] = cadd(t0, t2);
+      v[2] = csub(t0, t2);
+      v[1] = cadd_mi<INV>(t1, t3);
+      v[3] = csub_mi<INV>(t1, t3);
+    }
   }
 };
 
-template <bool INV, typename T2> struct Dft<8, INV, T2> {
+template <bool INV, typename T2, int NZ> struct Dft<8, INV, T2, NZ> {
   static __host__ __device__ __forceinline__ void run(T2* v) {
-    typedef decltype(v[0].x) T;
+    typedef typename CxTraits<T2>::T T;
+    typedef typename CxTraits<T2>::W W;
+    constexpr int NE = (NZ + 1) / 2, NO = NZ / 2;
     const T h = (T)0.7071067811865475244008444;
-    T2 e[4] = {v[0], v[2], v[4], v[6]};
-    T2 o[4] = {v[1], v[3], v[5], v[7]};
-    Dft<4, INV, T2>::run(e);
-    Dft<4, INV, T2>::run(o);
-    // o[k] *= w8^k, w8 = exp(-/+ i pi/4)
-    T2 w1, w3;
-    w1.x = h; w1.y = INV ? h : -h;
-    w3.x = -h; w3.y = INV ? h : -h;
-    o[1] = cmul(o[1], w1);
-    o[2] = mul_mi<INV>(o[2]);
-    o[3] = cmul(o[3], w3);
+    T2 e[4], o[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      v[k] = cadd(e[k], o[k]);
-      v[k + 4] = csub(e[k], o[k]);
+      if (k < NE) e[k] = v[2 * k];
+      if (k < NO) o[k] = v[2 * k + 1];
+    }
+    Dft<4, INV, T2, NE>::run(e);
+    if constexpr (NO == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) v[k] = v[k + 4] = e[k];
+    } else {
+      Dft<4, INV, T2, NO>::run(o);
+      // o[k] *= w8^k, w8 = exp(-/+ i pi/4)
+      W w1, w3;
+      w1.x = h; w1.y = INV ? h : -h;
+      w3.x = -h; w3.y = INV ? h : -h;
+      o[1] = cmul(o[1], w1);
+      o[3] = cmul(o[3], w3);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        v[k] = k == 2 ? cadd_mi<INV>(e[k], o[k]) : cadd(e[k], o[k]);
+        v[k + 4] = k == 2 ? csub_mi<INV>(e[k], o[k]) : csub(e[k], o[k]);
+      }
     }
   }
 };
@@ -170,42 +307,46 @@ template <> struct OddConst<7> {
   }
 };
 
-template <int R, bool INV, typename T2> struct DftOdd {
+template <int R, bool INV, typename T2, int NZ> struct DftOdd {
   // In place: the pair sums/differences replace v[1..R-1] before the outputs
   // are written back, so no second output array is live.
   static __host__ __device__ __forceinline__ void run(T2* v) {
-    typedef decltype(v[0].x) T;
+    typedef typename CxTraits<T2>::T T;
     constexpr int H = (R - 1) / 2;
     T2 t[H], u[H];
 #pragma unroll
     for (int m = 1; m <= H; m++) {
-      t[m - 1] = cadd(v[m], v[R - m]);
-      u[m - 1] = csub(v[m], v[R - m]);
+      if (R - m < NZ) {
+        t[m - 1] = cadd(v[m], v[R - m]);
+        u[m - 1] = csub(v[m], v[R - m]);
+      } else if (m < NZ) {
+        t[m - 1] = u[m - 1] = v[m];
+      }
     }
     const T2 a0 = v[0];
 #pragma unroll
-    for (int m = 0; m < H; m++) v[0] = cadd(v[0], t[m]);
+    for (int m = 0; m < H; m++)
+      if (m + 1 < NZ) v[0] = cadd(v[0], t[m]);
 #pragma unroll
     for (int k = 1; k <= H; k++) {
-      T2 re = a0, im;
-      im.x = 0; im.y = 0;
+      T2 re = a0, im = czero<T2>();
 #pragma unroll
       for (int m = 1; m <= H; m++) {
+        if (m >= NZ) continue;
         const T c = (T)OddConst<R>::c((m * k) % R);
         const T s = (T)OddConst<R>::s((m * k) % R);
         re = caxr(re, c, t[m - 1]);
         im = caxr(im, s, u[m - 1]);
       }
       // forward: y_k = re - i im, y_{R-k} = re + i im
-      const T2 mi = mul_mi<INV>(im);  // -i*im (fwd) or +i*im (inv)
-      v[k] = cadd(re, mi);
-      v[R - k] = csub(re, mi);
+      v[k] = cadd_mi<INV>(re, im);
+      v[R - k] = csub_mi<INV>(re, im);
     }
   }
 };
-template <bool INV, typename T2> struct Dft<3, INV, T2> : DftOdd<3, INV, T2> {};
-template <bool INV, typename T2> struct Dft<5, INV, T2> : DftOdd<5, INV, T2> {};
-template <bool INV, typename T2> struct Dft<7, INV, T2> : DftOdd<7, INV, T2> {};
+template <bool INV, typename T2, int NZ> struct Dft<3, INV, T2, NZ> : DftOdd<3, INV, T2, NZ> {};
+template <bool INV, typename T2, int NZ> struct Dft<5, INV, T2, NZ> : DftOdd<5, INV, T2, NZ> {};
+template <bool INV, typename T2, int NZ> struct Dft<7, INV, T2, NZ> : DftOdd<7, INV, T2, NZ> {};
 
 // ------------------------------------------------------------- stages ----
 // All kernels of the library share one dynamic shared-memory window; the FFT

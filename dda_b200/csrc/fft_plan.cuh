@@ -75,22 +75,21 @@ __host__ __device__ __forceinline__ void sfor(F&& f) {
 // multiply by exp(-/+ 2 pi i e / n) with compile-time e, n
 template <int E, int N, bool INV, typename T2>
 __host__ __device__ __forceinline__ T2 cmul_tw(T2 v) {
-  typedef decltype(v.x) T;
+  typedef typename CxTraits<T2>::T T;
   constexpr int e = ((E % N) + N) % N;
   if constexpr (e == 0) {
     return v;
   } else if constexpr (4 * e == N) {
     return mul_mi<INV>(v);  // exp(-i pi/2)
   } else if constexpr (2 * e == N) {
-    v.x = -v.x; v.y = -v.y;
-    return v;
+    return cneg(v);
   } else if constexpr (4 * e == 3 * N) {
     return mul_mi<!INV>(v);
   } else {
     constexpr CtCS cs = ct_cossin(-e, N);
     constexpr double c = (double)cs.c;
     constexpr double s = INV ? -(double)cs.s : (double)cs.s;
-    T2 w;
+    typename CxTraits<T2>::W w;
     w.x = (T)c;
     w.y = (T)s;
     return cmul(v, w);
@@ -106,26 +105,34 @@ __host__ __device__ constexpr int first_factor(int n) {
 // DFT of N values in registers, natural order in and out.  Base radices use
 // the cores of fft_engine.cuh; composite N = A*B splits as
 // X[k1 + A k2] = sum_n2 w_N^(n2 k1) w_B^(n2 k2) sum_n1 x[B n1 + n2] w_A^(n1 k1).
-template <int N, bool INV, typename T2, bool BASE = is_base_radix(N)>
+// NZ: inputs x[NZ..N) are zero padding (not read), as for Dft.
+template <int N, bool INV, typename T2, int NZ = N, bool BASE = is_base_radix(N)>
 struct DftN;
 
-template <int N, bool INV, typename T2>
-struct DftN<N, INV, T2, true> {
-  static __host__ __device__ __forceinline__ void run(T2* v) { Dft<N, INV, T2>::run(v); }
+template <bool INV, typename T2, int NZ>
+struct DftN<1, INV, T2, NZ, false> {
+  static __host__ __device__ __forceinline__ void run(T2*) {}
 };
 
-template <int N, bool INV, typename T2>
-struct DftN<N, INV, T2, false> {
+template <int N, bool INV, typename T2, int NZ>
+struct DftN<N, INV, T2, NZ, true> {
+  static __host__ __device__ __forceinline__ void run(T2* v) { Dft<N, INV, T2, NZ>::run(v); }
+};
+
+template <int N, bool INV, typename T2, int NZ>
+struct DftN<N, INV, T2, NZ, false> {
   static constexpr int A = first_factor(N);
   static constexpr int B = N / A;
+  static constexpr int NB = NZ < B ? NZ : B;  // columns with a non-zero input
   static __host__ __device__ __forceinline__ void run(T2* x) {
     T2 y[N];
-    sfor<0, B>([&](auto n2c) {
+    sfor<0, NB>([&](auto n2c) {
       constexpr int n2 = decltype(n2c)::value;
+      constexpr int K1 = (NZ - n2 + B - 1) / B;  // non-zero inputs of this column
       T2 t[A];
 #pragma unroll
-      for (int n1 = 0; n1 < A; n1++) t[n1] = x[B * n1 + n2];
-      DftN<A, INV, T2>::run(t);
+      for (int n1 = 0; n1 < K1; n1++) t[n1] = x[B * n1 + n2];
+      DftN<A, INV, T2, K1>::run(t);
       sfor<0, A>([&](auto k1c) {
         constexpr int k1 = decltype(k1c)::value;
         y[n2 + B * k1] = cmul_tw<n2 * k1, N, INV>(t[k1]);
@@ -135,8 +142,8 @@ struct DftN<N, INV, T2, false> {
     for (int k1 = 0; k1 < A; k1++) {
       T2 t[B];
 #pragma unroll
-      for (int n2 = 0; n2 < B; n2++) t[n2] = y[n2 + B * k1];
-      DftN<B, INV, T2>::run(t);
+      for (int n2 = 0; n2 < NB; n2++) t[n2] = y[n2 + B * k1];
+      DftN<B, INV, T2, NB>::run(t);
 #pragma unroll
       for (int k2 = 0; k2 < B; k2++) x[k1 + A * k2] = t[k2];
     }
@@ -188,13 +195,14 @@ template <int... Rs> struct Plan {
 // One stage of plan P applied to one butterfly: R = P::r[I], block length
 // L, stride S = L/R; v holds the R elements base + m*S.  Twiddle exponents
 // j*m*(N/L) index the length-N table tw (shared memory).
-template <typename P, int I, bool INV, typename T2>
+// NZ (forward stage 0): inputs v[NZ..R) are zero padding (not read).
+template <typename P, int I, bool INV, typename T2, int NZ = P::r[I]>
 __device__ __forceinline__ void butterfly(T2* v, int j, const T2* tw) {
   constexpr int R = P::r[I];
   constexpr int L = P::L(I);
   constexpr int TS = P::N / L;
   if constexpr (L == R) {  // last forward / first inverse stage: no twiddles
-    DftN<R, INV, T2>::run(v);
+    DftN<R, INV, T2, NZ>::run(v);
   } else if constexpr (INV) {
     if (j) {
 #pragma unroll
@@ -206,7 +214,7 @@ __device__ __forceinline__ void butterfly(T2* v, int j, const T2* tw) {
     }
     DftN<R, INV, T2>::run(v);
   } else {
-    DftN<R, INV, T2>::run(v);
+    DftN<R, INV, T2, NZ>::run(v);
     if (j) {
 #pragma unroll
       for (int m = 1; m < R; m++) v[m] = cmul(v[m], tw[j * m * TS]);

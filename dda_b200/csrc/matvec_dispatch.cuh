@@ -4,6 +4,7 @@
 #pragma once
 
 #include "matvec_kernels.cuh"
+#include "matvec_pass.cuh"
 #include "matvec_planned.cuh"
 #include "matvec_slot.cuh"
 #include "matvec_pair.cuh"
@@ -40,10 +41,21 @@ template <typename T> struct MvKernels {
   YrowsFn yrows = nullptr;  // split path
   ColsFn cols = nullptr;
   SlotFn slot = nullptr;    // cluster plane kernel for planes beyond shared memory
+  PassKernels<T, 1> pass1;  // y/z passes through the work buffer (matvec_pass.cuh)
+  PassKernels<T, 2> pass2;  // the same over pairs of right-hand sides (FP32)
   bool planned = false;
 };
 
 
+inline bool has_plan(int n) {
+  switch (n) {
+#define C(N) case N:
+    DDA_PASS_LENGTHS(C)
+#undef C
+    return true;
+    default: return false;
+  }
+}
 inline bool has_tuned_plan(int n) {
   switch (n) {
 #define C(N) case N:
@@ -110,15 +122,23 @@ void x_kernels(MvKernels<T>& k) {
   }
 }
 
-template <typename T, int NTX, bool M>
+// (S: part of the lengths, DDA_PASS_LENGTHS_<S>)
+#define DDA_BY_LENGTH(S, n)                  \
+  if constexpr (S == 0) {                    \
+    switch (n) { DDA_PASS_LENGTHS_0(C) }     \
+  } else if constexpr (S == 1) {             \
+    switch (n) { DDA_PASS_LENGTHS_1(C) }     \
+  } else if constexpr (S == 2) {             \
+    switch (n) { DDA_PASS_LENGTHS_2(C) }     \
+  } else {                                   \
+    switch (n) { DDA_PASS_LENGTHS_3(C) }     \
+  }
+template <typename T, int NTX, bool M, int S>
 void planned_x(MvKernels<T>& k, int gx) {
-  switch (gx) {
 #define C(N) \
   case N: x_kernels<T, NTX, typename PlanFor<N>::type, M>(k); break;
-    DDA_TUNED_LENGTHS(C)
+  DDA_BY_LENGTH(S, gx)
 #undef C
-    default: break;
-  }
 }
 
 template <typename T, int NTYZ, int NTC>
@@ -183,6 +203,24 @@ void planned_slot(MvKernels<T>& k, int gy, int gz, int by, int bz) {
   }
 }
 
+template <typename T, int S>
+void planned_pass(MvKernels<T>& k, int gy, int gz) {
+#define C(N)                                                                              \
+  case N:                                                                                 \
+    pass_z<T, 1, PlanFor<N>::type>(k.pass1);                                              \
+    if constexpr (sizeof(T) == 4) pass_z<T, 2, PlanFor<N>::type>(k.pass2);                \
+    break;
+  DDA_BY_LENGTH(S, gz)
+#undef C
+#define C(N)                                                                              \
+  case N:                                                                                 \
+    pass_y<T, 1, PlanFor<N>::type>(k.pass1);                                              \
+    if constexpr (sizeof(T) == 4) pass_y<T, 2, PlanFor<N>::type>(k.pass2);                \
+    break;
+  DDA_BY_LENGTH(S, gy)
+#undef C
+}
+
 template <typename T, int NTX, int NTYZ, int NTC>
 void generic_kernels(MvKernels<T>& k) {
   x_kernels<T, NTX, void, false>(k);
@@ -194,10 +232,10 @@ void generic_kernels(MvKernels<T>& k) {
 }
 
 // Entry points of the parts (defined in mv_inst.cu).
-void mv_part_x(MvKernels<float>& k, int gx);
-void mv_part_x(MvKernels<double>& k, int gx);
-void mv_part_xm(MvKernels<float>& k, int gx);
-void mv_part_xm(MvKernels<double>& k, int gx);
+template <int S> void mv_part_x(MvKernels<float>& k, int gx);
+template <int S> void mv_part_x(MvKernels<double>& k, int gx);
+template <int S> void mv_part_xm(MvKernels<float>& k, int gx);
+template <int S> void mv_part_xm(MvKernels<double>& k, int gx);
 void mv_part_split(MvKernels<float>& k, int gy, int gz, bool generic);
 void mv_part_split(MvKernels<double>& k, int gy, int gz, bool generic);
 void mv_part_fused(MvKernels<float>& k, int gy, int gz, int by, int bz);
@@ -206,9 +244,11 @@ void mv_part_slot(MvKernels<float>& k, int gy, int gz, int by, int bz);
 void mv_part_slot(MvKernels<double>& k, int gy, int gz, int by, int bz);
 void mv_part_pair(MvKernels<float>& k, int gy, int gz, int by, int bz);
 void mv_part_pair(MvKernels<double>& k, int gy, int gz, int by, int bz);
+template <int S> void mv_part_pass(MvKernels<float>& k, int gy, int gz);
+template <int S> void mv_part_pass(MvKernels<double>& k, int gy, int gz);
 
 // Kernel table of a context: compile-time-planned kernels for grid
-// (gx, gy, gz) and box extents by, bz when every edge is tuned, the
+// (gx, gy, gz) and box extents by, bz when every edge has a plan, the
 // runtime-planned ones otherwise.
 template <typename T>
 MvKernels<T> select_kernels(bool planned, int gx, int gy, int gz, int by, int bz) {
@@ -218,12 +258,13 @@ MvKernels<T> select_kernels(bool planned, int gx, int gy, int gz, int by, int bz
     mv_part_split(k, gy, gz, true);
     return k;
   }
-  mv_part_x(k, gx);
-  mv_part_xm(k, gx);
+  mv_part_x<0>(k, gx); mv_part_x<1>(k, gx); mv_part_x<2>(k, gx); mv_part_x<3>(k, gx);
+  mv_part_xm<0>(k, gx); mv_part_xm<1>(k, gx); mv_part_xm<2>(k, gx); mv_part_xm<3>(k, gx);
   mv_part_split(k, gy, gz, false);
   mv_part_fused(k, gy, gz, by, bz);
   mv_part_pair(k, gy, gz, by, bz);
   mv_part_slot(k, gy, gz, by, bz);
+  mv_part_pass<0>(k, gy, gz); mv_part_pass<1>(k, gy, gz); mv_part_pass<2>(k, gy, gz); mv_part_pass<3>(k, gy, gz);
   return k;
 }
 

@@ -67,12 +67,12 @@ __device__ __forceinline__ void load_dhat(const typename C2<T>::t* __restrict__ 
 
 // y = D x for the symmetric 3x3 matrix (xx, xy, xz, yy, yz, zz)
 // (Math/SymMatrix3.hpp:86-92).
-template <typename T2>
-__device__ __forceinline__ void dmul(const T2 d[6], T2& a, T2& b, T2& c) {
-  T2 x = a, y = b, z = c;
-  a = cadd(cadd(cmul(d[0], x), cmul(d[1], y)), cmul(d[2], z));
-  b = cadd(cadd(cmul(d[1], x), cmul(d[3], y)), cmul(d[4], z));
-  c = cadd(cadd(cmul(d[2], x), cmul(d[4], y)), cmul(d[5], z));
+template <typename V, typename W>
+__device__ __forceinline__ void dmul(const W d[6], V& a, V& b, V& c) {
+  const V x = a, y = b, z = c;
+  a = cfma(cfma(cmul(x, d[0]), d[1], y), d[2], z);
+  b = cfma(cfma(cmul(x, d[1]), d[3], y), d[4], z);
+  c = cfma(cfma(cmul(x, d[2]), d[4], y), d[5], z);
 }
 
 // True when right-hand side b needs no work: solved or failed, or (mvskip)

@@ -20,46 +20,117 @@
 
 namespace dda {
 
-// Grid lengths with compile-time plans, and those whose kx plane the fused
-// plane kernel k_yz_p handles (y and z both of that length).
+// Grid lengths with plane kernels in y and z (k_yz_p, k_yz_pair, k_yz_slot),
+// which dda_choose_grid rounds to, and those whose kx plane one CTA of k_yz_p
+// handles.
 #define DDA_TUNED_LENGTHS(X)                                                                               \
   X(32) X(48) X(56) X(64) X(80) X(96) X(100) X(112) X(120) X(128) X(144) X(160) X(168) X(192) X(200) X(224) \
   X(240) X(256) X(288) X(320) X(384) X(512)
 #define DDA_FUSED_LENGTHS(X) X(32) X(48) X(56) X(64) X(80) X(96) X(100) X(112) X(120) X(128)
 
-// Tuned plans: a large first radix and a last radix of at most 8, so the
-// fused last stage holds 3 x R_last complex values per thread.
+// Lengths with compile-time plans for the x passes and for the y/z passes of
+// matvec_pass.cuh, axis by axis: every even 2,3,5,7-smooth length from 8 to 512,
+// all that the reference's grid rule gives there, in four parts that compile
+// separately.
+#define DDA_PASS_LENGTHS_0(X) \
+  X(8) X(10) X(12) X(14) X(16) X(18) X(20) X(24) X(28) X(30) X(32) X(36) X(40) X(42) X(48) X(50) X(54) \
+  X(56) X(60) X(64) X(70) X(72)
+#define DDA_PASS_LENGTHS_1(X) \
+  X(80) X(84) X(90) X(96) X(98) X(100) X(108) X(112) X(120) X(126) X(128) X(140) X(144) X(150) X(160)
+#define DDA_PASS_LENGTHS_2(X) \
+  X(162) X(168) X(180) X(192) X(196) X(200) X(210) X(216) X(224) X(240) X(250) X(252) X(256)
+#define DDA_PASS_LENGTHS_3(X) \
+  X(270) X(280) X(288) X(294) X(300) X(320) X(324) X(336) X(350) X(360) X(378) X(384) X(392) X(400) X(420) \
+  X(432) X(448) X(450) X(480) X(486) X(490) X(500) X(504) X(512)
+#define DDA_PASS_LENGTHS(X) \
+  DDA_PASS_LENGTHS_0(X) DDA_PASS_LENGTHS_1(X) DDA_PASS_LENGTHS_2(X) DDA_PASS_LENGTHS_3(X)
+
+// Plans: a large first radix and a last radix of at most 8, so the fused last
+// y stage holds 3 x R_last complex values per thread; two stages up to 240
+// (in the row kernel a stage more costs half as much again), three beyond.
 template <int N> struct PlanFor { typedef void type; };
+template <> struct PlanFor<8> { typedef Plan<2, 4> type; };
+template <> struct PlanFor<10> { typedef Plan<2, 5> type; };
+template <> struct PlanFor<12> { typedef Plan<3, 4> type; };
+template <> struct PlanFor<14> { typedef Plan<2, 7> type; };
+template <> struct PlanFor<16> { typedef Plan<4, 4> type; };
+template <> struct PlanFor<18> { typedef Plan<6, 3> type; };
+template <> struct PlanFor<20> { typedef Plan<5, 4> type; };
+template <> struct PlanFor<24> { typedef Plan<6, 4> type; };
+template <> struct PlanFor<28> { typedef Plan<7, 4> type; };
+template <> struct PlanFor<30> { typedef Plan<6, 5> type; };
 template <> struct PlanFor<32> { typedef Plan<4, 8> type; };
+template <> struct PlanFor<36> { typedef Plan<6, 6> type; };
+template <> struct PlanFor<40> { typedef Plan<8, 5> type; };
+template <> struct PlanFor<42> { typedef Plan<6, 7> type; };
 template <> struct PlanFor<48> { typedef Plan<6, 8> type; };
+template <> struct PlanFor<50> { typedef Plan<10, 5> type; };
+template <> struct PlanFor<54> { typedef Plan<9, 6> type; };
 template <> struct PlanFor<56> { typedef Plan<7, 8> type; };
+template <> struct PlanFor<60> { typedef Plan<10, 6> type; };
 template <> struct PlanFor<64> { typedef Plan<8, 8> type; };
+template <> struct PlanFor<70> { typedef Plan<10, 7> type; };
+template <> struct PlanFor<72> { typedef Plan<12, 6> type; };
 template <> struct PlanFor<80> { typedef Plan<10, 8> type; };
+template <> struct PlanFor<84> { typedef Plan<12, 7> type; };
+template <> struct PlanFor<90> { typedef Plan<15, 6> type; };
 template <> struct PlanFor<96> { typedef Plan<12, 8> type; };
+template <> struct PlanFor<98> { typedef Plan<14, 7> type; };
 template <> struct PlanFor<100> { typedef Plan<20, 5> type; };
+template <> struct PlanFor<108> { typedef Plan<18, 6> type; };
 template <> struct PlanFor<112> { typedef Plan<14, 8> type; };
 template <> struct PlanFor<120> { typedef Plan<15, 8> type; };
+template <> struct PlanFor<126> { typedef Plan<18, 7> type; };
 template <> struct PlanFor<128> { typedef Plan<16, 8> type; };
+template <> struct PlanFor<140> { typedef Plan<20, 7> type; };
 template <> struct PlanFor<144> { typedef Plan<18, 8> type; };
+template <> struct PlanFor<150> { typedef Plan<25, 6> type; };
 template <> struct PlanFor<160> { typedef Plan<20, 8> type; };
+template <> struct PlanFor<162> { typedef Plan<27, 6> type; };
 template <> struct PlanFor<168> { typedef Plan<21, 8> type; };
+template <> struct PlanFor<180> { typedef Plan<30, 6> type; };
 template <> struct PlanFor<192> { typedef Plan<24, 8> type; };
+template <> struct PlanFor<196> { typedef Plan<28, 7> type; };
 template <> struct PlanFor<200> { typedef Plan<25, 8> type; };
+template <> struct PlanFor<210> { typedef Plan<30, 7> type; };
+template <> struct PlanFor<216> { typedef Plan<27, 8> type; };
 template <> struct PlanFor<224> { typedef Plan<28, 8> type; };
 template <> struct PlanFor<240> { typedef Plan<30, 8> type; };
+template <> struct PlanFor<250> { typedef Plan<10, 5, 5> type; };
+template <> struct PlanFor<252> { typedef Plan<12, 3, 7> type; };
 template <> struct PlanFor<256> { typedef Plan<8, 4, 8> type; };
+template <> struct PlanFor<270> { typedef Plan<9, 6, 5> type; };
+template <> struct PlanFor<280> { typedef Plan<10, 4, 7> type; };
 template <> struct PlanFor<288> { typedef Plan<6, 6, 8> type; };
+template <> struct PlanFor<294> { typedef Plan<14, 3, 7> type; };
+template <> struct PlanFor<300> { typedef Plan<12, 5, 5> type; };
 template <> struct PlanFor<320> { typedef Plan<5, 8, 8> type; };
+template <> struct PlanFor<324> { typedef Plan<9, 6, 6> type; };
+template <> struct PlanFor<336> { typedef Plan<12, 4, 7> type; };
+template <> struct PlanFor<350> { typedef Plan<10, 5, 7> type; };
+template <> struct PlanFor<360> { typedef Plan<12, 6, 5> type; };
+template <> struct PlanFor<378> { typedef Plan<9, 6, 7> type; };
 template <> struct PlanFor<384> { typedef Plan<6, 8, 8> type; };
-template <> struct PlanFor<512> { typedef Plan<8, 8, 8> type; };
+template <> struct PlanFor<392> { typedef Plan<14, 4, 7> type; };
+template <> struct PlanFor<400> { typedef Plan<16, 5, 5> type; };
+template <> struct PlanFor<420> { typedef Plan<12, 5, 7> type; };
+template <> struct PlanFor<432> { typedef Plan<12, 6, 6> type; };
+template <> struct PlanFor<448> { typedef Plan<16, 4, 7> type; };
+template <> struct PlanFor<450> { typedef Plan<15, 6, 5> type; };
+template <> struct PlanFor<480> { typedef Plan<16, 6, 5> type; };
+template <> struct PlanFor<486> { typedef Plan<9, 9, 6> type; };
+template <> struct PlanFor<490> { typedef Plan<14, 5, 7> type; };
+template <> struct PlanFor<500> { typedef Plan<20, 5, 5> type; };
+template <> struct PlanFor<504> { typedef Plan<12, 6, 7> type; };
+template <> struct PlanFor<512> { typedef Plan<16, 4, 8> type; };
 
-// Radices of the tuned plan for n (host side), empty when there is none.
-inline std::vector<int> tuned_radices(int n) {
+// Radices of the compile-time plan for n (host side), empty when there is none.
+inline std::vector<int> plan_radices(int n) {
   auto get = [](auto p) { return std::vector<int>(std::begin(decltype(p)::r), std::end(decltype(p)::r)); };
   switch (n) {
 #define C(N) \
   case N: return get(typename PlanFor<N>::type());
-    DDA_TUNED_LENGTHS(C)
+    DDA_PASS_LENGTHS(C)
 #undef C
     default: return {};
   }

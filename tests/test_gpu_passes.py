@@ -1,0 +1,51 @@
+"""The y/z passes as three kernels (matvec_pass.cuh) and the planned x passes
+against the oracle, at FP64 1e-12 and FP32 2e-6 relative in the 2-norm as for
+the other matvec paths: two- and three-stage plans on every axis, odd and even
+first radices, last radices 2 to 8, boxes of half the grid and of less, one
+right-hand side (W = 1), a pair, and a pair with an idle lane."""
+import numpy as np
+import pytest
+
+from tests.pairs import Pair, rel
+
+pytestmark = pytest.mark.gpu
+
+BOXES = {
+    (4, 4, 4): (8, 8, 8),
+    (5, 7, 9): (10, 14, 18),
+    (9, 15, 27): (18, 30, 54),
+    (11, 13, 11): (24, 28, 24),        # less than half of every edge
+    (35, 49, 21): (70, 98, 42),
+    (33, 45, 81): (70, 90, 162),       # odd first radices
+    (140, 6, 5): (280, 12, 10),        # three stages along x
+    (6, 125, 8): (12, 250, 16),        # ... y
+    (5, 6, 150): (10, 12, 300),        # ... z
+    (8, 110, 128): (16, 224, 256),
+    (4, 63, 126): (8, 126, 252),
+}
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-12), ("fp32", 2e-6)])
+@pytest.mark.parametrize("box", list(BOXES))
+def test_passes_match_oracle(box, prec, tol):
+    rng = np.random.default_rng(box[0])
+    z, y, x = np.meshgrid(*[np.arange(n) for n in box[::-1]], indexing="ij")
+    keep = rng.random(x.shape) < 0.7
+    keep[0, 0, 0] = keep[-1, -1, -1] = True  # the box's corners
+    pos = np.stack([x[keep], y[keep], z[keep]], axis=1).astype(np.uint32)
+    mat = (rng.random(len(pos)) < 0.4).astype(np.uint8)
+    pr = Pair("arrays", (pos, mat, "0.1um"), [1.5 + 0.1j, 1.3 + 0.02j], "1.1um", prec, max_rhs=3)
+    assert pr.p.grid == BOXES[box] and pr.mv.passes
+    xs = [pr.rand_vec(40 + r) for r in range(3)]
+    want = []
+    for r, pol in enumerate((1, 2, 1)):
+        pr.set_cc((0.36, 0.48, 0.8) if r else (0, 0, 1), pol, "ldr", rhs=r)
+        want.append(pr.op.matvec(xs[r]))
+    n = pr.p.vec_size
+    three = pr.mv.apply(np.concatenate(xs)).reshape(3, n)
+    for r in range(3):
+        assert rel(three[r], want[r]) < tol, r
+    # alone and as a pair: the same bits
+    assert np.array_equal(pr.mv.apply(xs[0]), three[0])
+    assert np.array_equal(pr.mv.apply(np.concatenate(xs[:2])).reshape(2, n), three[:2])
+    pr.mv.close()
