@@ -162,6 +162,81 @@ __device__ __forceinline__ A2 xpre_value(int op, int first, A2 p, A2 v1, A2 v2, 
   }
 }
 
+// ---- the x transform of a tile with a compile-time plan ---------------------
+// The tile's lines fill [0, bx) of their rows (pitch apart, at soff); the
+// grid is at least twice the box, so of a stage-0 butterfly's inputs those
+// with m >= (R + 1) / 2 are zero padding, which is neither stored nor read,
+// and of the inverse's outputs those are dropped.  The last forward stage
+// leaves its outputs in registers and stores them to the x spectrum, the
+// first inverse stage reads its inputs from there: with neighbouring lanes on
+// neighbouring lines each access covers a run of lines, and the tile passes
+// through shared memory once less each way.  These passes are bound by issue
+// (56 % of it) and the shared-memory pipe, so that is time: forward / inverse
+// of the 128-rhs spheroid 1.29 -> 1.03 / 1.57 -> 1.37 ms, of the two-rhs box
+// 22.5 -> 19.6 / 28.7 -> 25.4 us.
+template <typename T, typename P, int G>
+__device__ __forceinline__ void x_lines_fwd(int soff, int nl, int pitch, int bx, typename C2<T>::t* __restrict__ out,
+                                            size_t kstride) {
+  typedef typename C2<T>::t T2;
+  constexpr int K = P::K, R = P::r[0], S0 = P::N / R, NZ = (R + 1) / 2, RL = P::r[K - 1], NB = P::N / RL;
+  T2* s = smem_at<T>(0);
+  for (int b = threadIdx.x; b < nl * S0; b += G) {
+    const int j = b / nl, l = b - j * nl;
+    const int base = soff + l * pitch + j;
+    T2 v[R];
+#pragma unroll
+    for (int m = 0; m < NZ; m++) v[m] = j + m * S0 < bx ? s[base + m * S0] : czero<T2>();
+    butterfly<P, 0, false, T2, NZ>(v, j, s);
+#pragma unroll
+    for (int m = 0; m < R; m++) s[base + m * S0] = v[m];
+  }
+  __syncthreads();
+  pstages<T, P, false, G, 1, K - 1>(soff, nl, pitch, 1, 0, threadIdx.x);
+  for (int b = threadIdx.x; b < nl * NB; b += G) {
+    const int t = b / nl, l = b - t * nl;
+    const int base = soff + l * pitch + t * RL;
+    T2 v[RL];
+#pragma unroll
+    for (int m = 0; m < RL; m++) v[m] = s[base + m];
+    DftN<RL, false, T2>::run(v);
+    T2* o = out + (size_t)(t * RL) * kstride + l;
+#pragma unroll
+    for (int m = 0; m < RL; m++) o[m * kstride] = v[m];
+  }
+}
+template <typename T, typename P, int G>
+__device__ __forceinline__ void x_lines_inv(int soff, int nl, int pitch, int bx,
+                                            const typename C2<T>::t* __restrict__ in, size_t kstride) {
+  typedef typename C2<T>::t T2;
+  constexpr int K = P::K, R = P::r[0], S0 = P::N / R, NZ = (R + 1) / 2, RL = P::r[K - 1], NB = P::N / RL;
+  T2* s = smem_at<T>(0);
+  for (int b = threadIdx.x; b < nl * NB; b += G) {
+    const int t = b / nl, l = b - t * nl;
+    const T2* i = in + (size_t)(t * RL) * kstride + l;
+    T2 v[RL];
+#pragma unroll
+    for (int m = 0; m < RL; m++) v[m] = i[m * kstride];
+    DftN<RL, true, T2>::run(v);
+    const int base = soff + l * pitch + t * RL;
+#pragma unroll
+    for (int m = 0; m < RL; m++) s[base + m] = v[m];
+  }
+  __syncthreads();
+  pstages<T, P, true, G, 1, K - 1>(soff, nl, pitch, 1, 0, threadIdx.x);
+  for (int b = threadIdx.x; b < nl * S0; b += G) {
+    const int j = b / nl, l = b - j * nl;
+    const int base = soff + l * pitch + j;
+    T2 v[R];
+#pragma unroll
+    for (int m = 0; m < R; m++) v[m] = s[base + m * S0];
+    butterfly<P, 0, true>(v, j, s);
+#pragma unroll
+    for (int m = 0; m < NZ; m++)
+      if (j + m * S0 < bx) s[base + m * S0] = v[m];
+  }
+  __syncthreads();
+}
+
 // ------------------------------------------------------------ k_xfwd ----
 // grid (ceil(nlines/tl), 3, nrhs).  PX: compile-time plan of the x
 // transform, or void for the runtime-planned engine.  A2: the vectors'
@@ -190,7 +265,12 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 3) k_xfwd(const A2* _
   stage_twiddles<T, NT>(0, px);
   for (int i = threadIdx.x; i < g.nmat; i += NT) scc[i] = ccs[((size_t)b * g.nmat + i) * 3 + c];
   for (int i = threadIdx.x; i <= nl; i += NT) soff[i] = line_off[L0 + i];
-  for (int i = threadIdx.x; i < nl * g.pitchx; i += NT) sm[i] = czero<T2>();
+  if constexpr (std::is_void<PX>::value) {
+    for (int i = threadIdx.x; i < nl * g.pitchx; i += NT) sm[i] = czero<T2>();
+  } else {
+    for (int l = threadIdx.x >> 5; l < nl; l += NT / 32)
+      for (int x = threadIdx.x & 31; x < g.bx; x += 32) sm[l * g.pitchx + x] = czero<T2>();
+  }
   __syncthreads();
   // the tile's dipoles are one contiguous CSR range: every thread takes
   // entries of it independently, so many loads are in flight at once
@@ -258,11 +338,14 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 3) k_xfwd(const A2* _
   if (PRE && blockIdx.x == 0)
     for (int i = g.nv + threadIdx.x; i < g.nvs; i += NT) po[i] = czero<A2>();
   __syncthreads();
-  if constexpr (std::is_void<PX>::value) fft_lines<T, NT, false>(toff, nl, g.pitchx, 1, false, px, 0);
-  else plines<T, PX, NT, false>(toff, nl, g.pitchx, 1, 0);
   T2* out = xhat + ((size_t)b * g.Gx * 3 + c) * g.nlines + L0;
   const size_t kstride = (size_t)3 * g.nlines;
-  for (TileWalk<NT> w(nl); w.kx < g.Gx; w.next(nl)) out[w.kx * kstride + w.l] = sm[w.l * g.pitchx + w.kx];
+  if constexpr (std::is_void<PX>::value) {
+    fft_lines<T, NT, false>(toff, nl, g.pitchx, 1, false, px, 0);
+    for (TileWalk<NT> w(nl); w.kx < g.Gx; w.next(nl)) out[w.kx * kstride + w.l] = sm[w.l * g.pitchx + w.kx];
+  } else {
+    x_lines_fwd<T, PX, NT>(toff, nl, g.pitchx, g.bx, out, kstride);
+  }
   if (PRE && pre.step.op != KOP_NONE) {
     RedSums tot;
     const int part = blockIdx.y * gridDim.x + blockIdx.x;
@@ -302,25 +385,29 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 3) k_xinv(const A2* _
   for (int i = threadIdx.x; i <= nl; i += NT) soff[i] = line_off[L0 + i];
   const T2* in = xhat + ((size_t)b * g.Gx * 3 + c) * g.nlines + L0;
   const size_t kstride = (size_t)3 * g.nlines;
-  for (TileWalk<NT> w(nl); w.kx < g.Gx;) {
-    T2 v[kXBatch];
-    int o[kXBatch];  // shared offset, -1 past the tile
-#pragma unroll
-    for (int u = 0; u < kXBatch; u++) {
-      o[u] = -1;
-      if (w.kx < g.Gx) {
-        v[u] = in[w.kx * kstride + w.l];
-        o[u] = w.l * g.pitchx + w.kx;
+  if constexpr (std::is_void<PX>::value) {
+    for (TileWalk<NT> w(nl); w.kx < g.Gx;) {
+      T2 v[kXBatch];
+      int o[kXBatch];  // shared offset, -1 past the tile
+  #pragma unroll
+      for (int u = 0; u < kXBatch; u++) {
+        o[u] = -1;
+        if (w.kx < g.Gx) {
+          v[u] = in[w.kx * kstride + w.l];
+          o[u] = w.l * g.pitchx + w.kx;
+        }
+        w.next(nl);
       }
-      w.next(nl);
+  #pragma unroll
+      for (int u = 0; u < kXBatch; u++)
+        if (o[u] >= 0) sm[o[u]] = v[u];
     }
-#pragma unroll
-    for (int u = 0; u < kXBatch; u++)
-      if (o[u] >= 0) sm[o[u]] = v[u];
+    __syncthreads();
+    fft_lines<T, NT, true>(toff, nl, g.pitchx, 1, false, px, 0);
+  } else {
+    __syncthreads();
+    x_lines_inv<T, PX, NT>(toff, nl, g.pitchx, g.bx, in, kstride);
   }
-  __syncthreads();
-  if constexpr (std::is_void<PX>::value) fft_lines<T, NT, true>(toff, nl, g.pitchx, 1, false, px, 0);
-  else plines<T, PX, NT, true>(toff, nl, g.pitchx, 1, 0);
   const size_t voff = ((size_t)b * 3 + c) * g.nvs;
   const A2* a = arg + voff;
   A2* r = res + voff;
