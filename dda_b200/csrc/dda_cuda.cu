@@ -233,7 +233,8 @@ template <typename T> struct Engine {
   void* pbuf = nullptr;       // work buffer of the y/z passes (matvec_pass.cuh)
   size_t pbuf_bytes = 0;
   bool pass = false;          // the y/z passes exist for this grid
-  T2* vec[10] = {};    // Krylov vectors [max_rhs][3 nvs]
+  T2* vec[10] = {};    // Krylov vectors [max_rhs][3 nvs], parts of one allocation
+  size_t vec_bytes = 0;  // of that allocation
   T2* io = nullptr;    // host-API staging [max_rhs][3 nvs]
   T2* xo = nullptr;    // MIXED, FP64 engine: refined solution x and b = sqrt(cc) Einc
   T2* bo = nullptr;
@@ -257,8 +258,7 @@ template <typename T> struct Engine {
     for (void* p : {(void*)dc, (void*)ccs, (void*)xhat, (void*)zbuf, (void*)io, (void*)slots, (void*)order,
                     (void*)xo, (void*)bo, pbuf})
       if (p) cudaFreeAsync(p, s);
-    for (auto& v : vec)
-      if (v) cudaFreeAsync(v, s);
+    if (vec[0]) cudaFreeAsync(vec[0], s);
     dc = ccs = xhat = zbuf = io = slots = xo = bo = nullptr;
     pbuf = nullptr;
     order = nullptr;
@@ -663,11 +663,12 @@ template <typename T> void setup_engine(dda_ctx* c) {
   // a MIXED context runs its Krylov vectors in FP64 and only the matvec's
   // convolution in FP32: the FP32 engine needs one input buffer and io
   const bool conv_engine = c->precision == DDA_PREC_MIXED && sizeof(T) == 4;
-  for (int i = 0; i < 10; i++) {
-    if (conv_engine && i > 0) break;
-    e.vec[i] = (T2*)dalloc<T>(vbytes);
-    CK(cudaMemsetAsync(e.vec[i], 0, vbytes, c->stream));
-  }
+  const int nvec = conv_engine ? 1 : 10;
+  const size_t vpitch = (vbytes + 255) / 256 * 256;
+  e.vec_bytes = nvec * vpitch;
+  e.vec[0] = (T2*)dalloc<T>(e.vec_bytes);
+  CK(cudaMemsetAsync(e.vec[0], 0, e.vec_bytes, c->stream));
+  for (int i = 1; i < nvec; i++) e.vec[i] = (T2*)((char*)e.vec[0] + i * vpitch);
   e.io = (T2*)dalloc<T>(vbytes);
   if (c->precision == DDA_PREC_MIXED && sizeof(T) == 8) {
     e.xo = (T2*)dalloc<T>(vbytes);
@@ -2221,7 +2222,7 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
     // vectors: 10 Krylov + io; MIXED keeps two more in FP64 (x, b) and only
     // the matvec input and io in FP32
     const long long nvec = precision != DDA_PREC_MIXED ? 11 : s == 16 ? 13 : 2;
-    e += R * nmat * 3 * s + R * Gx * 3 * nl * s + nvec * R * 3 * nvs * s;
+    e += R * nmat * 3 * s + R * Gx * 3 * nl * s + nvec * (R * 3 * nvs * s + 255);
     const long long q = 3 * by + ((3 * by) % 2 == 0 ? 1 : 0);
     const long long smem_yz = (Gz + Gy + Gz * q + 3 * (Gy + 1)) * s;
     bool fused_len = false;
@@ -2284,17 +2285,19 @@ int dda_profile_matvec(dda_ctx* ctx, int nrhs, int reps, double* ms) {
 }  // extern "C"
 
 namespace {
-template <typename T>
-void far_field_t(dda_ctx* c, int nrhs, const double* pol, long long ndir, const double* dirs, double* out) {
-  typedef typename C2<T>::t T2;
-  Engine<T>& e = eng<T>(c);
-  const size_t n = (size_t)nrhs * 3 * c->g.nvs;
-  if (pol) host_to_engine<T>(c, pol, e.io, n);
-  double* ddirs = nullptr;
-  double2* dout = nullptr;
-  CK(cudaMallocAsync(&ddirs, ndir * 3 * sizeof(double), c->stream));
-  CK(cudaMallocAsync(&dout, (size_t)ndir * nrhs * 3 * sizeof(double2), c->stream));
-  CK(cudaMemcpyAsync(ddirs, dirs, ndir * 3 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+// The far field of e.io: k_farfield for a few directions, whose lines are
+// then the only parallelism, or where the x phases of 32 directions do not
+// fit shared memory; else k_ff_part, directions on the lanes.
+// Threshold: 40^3 sphere, FP64, both polarisations: 31 directions 177 us with
+// k_farfield, 32 with k_ff_part 128 (5 551: 1 653 -> 745); with at most one
+// line per thread (14 x 14 x 10) k_farfield is as fast up to 56 (50 to 56 us).
+// Two directions per lane help where a lane has one right-hand side (40^3,
+// FP32, 5 551 directions: 471 -> 418 us; 1 024: 196 -> 178), not two, which
+// give a read 24 FMAs already (744 and 770).
+constexpr int kFfFew = 32, kFfTwo = 1024;
+constexpr size_t kFfPartBytes = (size_t)64 << 20;  // of a request that allocates
+
+FfGeom far_field_geom(const dda_ctx* c) {
   FfGeom g;
   g.nv = c->g.nv;
   g.nvs = c->g.nvs;
@@ -2307,17 +2310,84 @@ void far_field_t(dda_ctx* c, int nrhs, const double* pol, long long ndir, const 
   g.ox = -((double)c->g.bx - 1) / 2 * c->grid_unit;
   g.oy = -((double)c->g.by - 1) / 2 * c->grid_unit;
   g.oz = -((double)c->g.bz - 1) / 2 * c->grid_unit;
+  return g;
+}
+
+template <typename T>
+void far_field_few(dda_ctx* c, int nrhs, const double* ddirs, long long ndir, double2* dout) {
+  const FfGeom g = far_field_geom(c);
   constexpr int DB = 4, NT = 256;
   const size_t smem = (size_t)DB * g.bx * sizeof(double2);
   if (smem > kSmemMax) throw DdaError(DDA_ERR_UNSUPPORTED, "box too long for the far-field tables");
   CK(allow_smem((const void*)k_farfield<T, NT, DB>));
   k_farfield<T, NT, DB><<<dim3((unsigned)((ndir + DB - 1) / DB), nrhs), NT, smem, c->stream>>>(
-      e.io, c->line_off, c->dip, c->perm, ddirs, (int)ndir, g, dout);
+      eng<T>(c).io, c->line_off, c->dip, c->perm, ddirs, (int)ndir, g, dout);
   CK(cudaGetLastError());
   c->launches++;
+}
+
+// part: room for part_bytes of partial sums.
+template <typename T, int NR, int DL>
+void far_field_many(dda_ctx* c, int nrhs, const double* ddirs, long long ndir, double2* dout, double2* part,
+                    size_t part_bytes) {
+  const FfGeom g = far_field_geom(c);
+  const size_t smem = ff_part_smem<NR, DL>(g.bx), row = (size_t)nrhs * 3 * sizeof(double2);
+  CK(allow_smem((const void*)k_ff_part<T, NR, DL>));
+  int nsm = 148;
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+  const int zr = (nrhs + NR - 1) / NR, nd = 32 * DL;
+  // directions per launch and splits of the lines: about eight waves of CTAs,
+  // at least two lines per warp, within the room
+  const long long fit = std::max<long long>(1, (long long)(part_bytes / row));
+  const long long ctas = (std::min(ndir, fit) + nd - 1) / nd * zr;
+  long long splits = (16LL / DL * nsm + ctas - 1) / ctas;
+  splits = std::max<long long>(1, std::min<long long>({splits, 64, g.nlines / (2 * (kNtFf / 32)), fit / nd}));
+  const long long block = std::min<long long>(ndir, fit / splits);
+  for (long long d0 = 0; d0 < ndir; d0 += block) {
+    const int n = (int)std::min(block, ndir - d0);
+    k_ff_part<T, NR, DL><<<dim3((n + nd - 1) / nd, (unsigned)splits, zr), kNtFf, smem, c->stream>>>(
+        eng<T>(c).io, c->line_off, c->dip, c->perm, ddirs + 3 * d0, n, nrhs, g, part);
+    k_ff_combine<<<(unsigned)(((long long)n * nrhs + 127) / 128), 128, 0, c->stream>>>(
+        part, (int)splits, ddirs + 3 * d0, n, nrhs, g, dout + (size_t)d0 * nrhs * 3);
+    c->launches += 2;
+  }
+  CK(cudaGetLastError());
+}
+
+template <typename T>
+void far_field_t(dda_ctx* c, int nrhs, const double* pol, long long ndir, const double* dirs, double* out) {
+  typedef typename C2<T>::t T2;
+  Engine<T>& e = eng<T>(c);
+  const size_t n = (size_t)nrhs * 3 * c->g.nvs;
+  if (pol) host_to_engine<T>(c, pol, e.io, n);
+  // directions, fields and partial sums live in the Krylov vectors, which hold
+  // nothing between solves (a call's own allocations cost more than small far
+  // fields: the pool returns them at the next synchronisation); a request
+  // beyond them allocates
+  const size_t dbytes = ((size_t)ndir * 3 * sizeof(double) + 255) / 256 * 256;
+  const size_t obytes = ((size_t)ndir * nrhs * 3 * sizeof(double2) + 255) / 256 * 256;
+  const bool many = ndir >= (c->g.nlines > 256 ? kFfFew : 2 * kFfFew) && ff_part_smem<2, 1>(c->g.bx) <= kSmemMax;
+  const bool two = nrhs == 1 && ndir >= kFfTwo && ff_part_smem<1, 2>(c->g.bx) <= kSmemMax;
+  const size_t least = many ? std::min(obytes, kFfPartBytes) : 0;  // one split of the lines
+  char* buf = (char*)e.vec[0];
+  size_t room = e.vec_bytes;
+  void* temp = nullptr;
+  if (dbytes + obytes + least > room) {
+    room = dbytes + obytes + least;
+    CK(cudaMallocAsync(&temp, room, c->stream));
+    buf = (char*)temp;
+  }
+  double* ddirs = (double*)buf;
+  double2* dout = (double2*)(buf + dbytes);
+  double2* part = (double2*)(buf + dbytes + obytes);
+  const size_t part_bytes = room - dbytes - obytes;
+  CK(cudaMemcpyAsync(ddirs, dirs, ndir * 3 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  if (!many) far_field_few<T>(c, nrhs, ddirs, ndir, dout);
+  else if (two) far_field_many<T, 1, 2>(c, nrhs, ddirs, ndir, dout, part, part_bytes);
+  else if (nrhs == 1) far_field_many<T, 1, 1>(c, nrhs, ddirs, ndir, dout, part, part_bytes);
+  else far_field_many<T, 2, 1>(c, nrhs, ddirs, ndir, dout, part, part_bytes);
   CK(cudaMemcpyAsync(out, dout, (size_t)ndir * nrhs * 3 * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaFreeAsync(ddirs, c->stream));
-  CK(cudaFreeAsync(dout, c->stream));
+  if (temp) CK(cudaFreeAsync(temp, c->stream));
   CK(cudaStreamSynchronize(c->stream));
 }
 
@@ -2359,31 +2429,11 @@ unsigned char* ff_scratch(int device) {
 
 template <typename T>
 void far_field_noalloc_t(dda_ctx* c, int nrhs, long long ndir, const double* dirs, double* out) {
-  Engine<T>& e = eng<T>(c);
   unsigned char* scratch = ff_scratch(c->device);
   double* ddirs = reinterpret_cast<double*>(scratch);
   double2* dout = reinterpret_cast<double2*>(scratch + ((ndir * 3 * sizeof(double) + 255) & ~(size_t)255));
   CK(cudaMemcpyAsync(ddirs, dirs, ndir * 3 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  FfGeom g;
-  g.nv = c->g.nv;
-  g.nvs = c->g.nvs;
-  g.by = c->g.by;
-  g.nlines = c->g.nlines;
-  g.bx = c->g.bx;
-  g.kd = c->kd;
-  g.k = c->kd / c->grid_unit;
-  // DipoleGeometry::moveToCenter (DDA/DipoleGeometry.cpp:75-80)
-  g.ox = -((double)c->g.bx - 1) / 2 * c->grid_unit;
-  g.oy = -((double)c->g.by - 1) / 2 * c->grid_unit;
-  g.oz = -((double)c->g.bz - 1) / 2 * c->grid_unit;
-  constexpr int DB = 4, NT = 256;
-  const size_t smem = (size_t)DB * g.bx * sizeof(double2);
-  if (smem > kSmemMax) throw DdaError(DDA_ERR_UNSUPPORTED, "box too long for the far-field tables");
-  CK(allow_smem((const void*)k_farfield<T, NT, DB>));
-  k_farfield<T, NT, DB><<<dim3((unsigned)((ndir + DB - 1) / DB), nrhs), NT, smem, c->stream>>>(
-      e.io, c->line_off, c->dip, c->perm, ddirs, (int)ndir, g, dout);
-  CK(cudaGetLastError());
-  c->launches++;
+  far_field_few<T>(c, nrhs, ddirs, ndir, dout);
   CK(cudaMemcpyAsync(out, dout, (size_t)ndir * nrhs * 3 * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
 }
