@@ -300,8 +300,8 @@ struct dda_ctx {
   double* hist = nullptr;
   long long hist_cap = 0;
   long long launches = 0;  // kernels this context has launched
-  // instantiated graphs of one solver round, per (solver, nrhs, precision):
-  // the round's kernel arguments are the context's fixed buffers
+  // instantiated graphs of two solver iterations, per (solver, nrhs, precision):
+  // their kernel arguments are the context's fixed buffers
   struct RoundGraph {
     int solver, nrhs, tsize;
     cudaGraphExec_t g;
@@ -1332,6 +1332,38 @@ bool check_gap(dda_ctx* c, int nrhs, double2* X, double2* B, double2* tmp, const
   return all;
 }
 
+// Iterations of the next round: `poll`, or fewer when every running right-hand
+// side is expected to converge within them.  A kernel whose right-hand sides
+// are all done still costs its launch (a BiCGStab iteration of the two-rhs box
+// 43 us of about 240), a look at the flags some 20 us.  The expectation is the
+// mean rate of the residual since the last look; a round is an even number of
+// iterations (RoundGraph), and rounds end on multiples of `poll` wherever they
+// are not cut short, so that what is done every so many iterations is done at
+// the same ones.
+struct RoundLength {
+  std::vector<double> last;
+  long long last_nr = 0;
+  RoundLength(const KrylovState* st, int nrhs) : last(nrhs, 0.0) {
+    for (int r = 0; r < nrhs; r++) last[r] = st[r].inprodR;
+  }
+  int update(const KrylovState* st, long long nr, int poll) {
+    const int full = poll - (int)(nr % poll);
+    double need = 0;
+    for (size_t r = 0; r < last.size(); r++) {
+      const KrylovState& k = st[r];
+      const double now = k.inprodR;
+      if (!k.done) {
+        const double rate = nr > last_nr && last[r] > now ? std::log(last[r] / now) / (double)(nr - last_nr) : 0.0;
+        need = std::max(need, rate > 0 && k.epsB > 0 ? std::log(now / k.epsB) / rate : (double)full);
+      }
+      last[r] = now;
+    }
+    last_nr = nr;
+    if (!(need < full)) return full;
+    return std::max(2, std::min(full, 2 * (int)std::ceil(need / 2)));
+  }
+};
+
 // Runs one solve of `nrhs` right-hand sides already set up in the engine
 // vectors (E = einc or B = b, S = start).  Per-rhs states end in c->st_host;
 // the solution x is left in engine vector 4.
@@ -1377,14 +1409,16 @@ void run_solve(dda_ctx* c, int solver, int nrhs, double eps, long long max_iter,
   CK(cudaMemcpyAsync(c->st, c->st_host, nrhs * sizeof(KrylovState), cudaMemcpyHostToDevice, c->stream));
   sv.solver_init(solver, b);
   long long nr = 0;
-  // The host looks at the convergence flags every `poll` iterations.  The
-  // first round (iterations 0..7 hold the solvers' first-iteration variants)
-  // is launched kernel by kernel; the second round is captured into a CUDA
-  // graph once and every later round replays it.  poll is even, so the
-  // buffers the solvers rotate on the host are back in the captured order
-  // after each round; all other kernel arguments are fixed pointers, and
-  // the kernels read their scalars and done flags from the device state.
-  const int poll = 8;
+  // The host looks at the convergence flags every `poll` iterations, or
+  // sooner when the residuals say that the solve ends sooner (RoundLength).
+  // The first round (iterations 0..7 hold the solvers' first-iteration
+  // variants) is launched kernel by kernel; after it two iterations are
+  // captured into a CUDA graph once and every later round replays it.  After
+  // two iterations the buffers the solvers rotate on the host are back in the
+  // captured order; all other kernel arguments are fixed pointers, and the
+  // kernels read their scalars and done flags from the device state.
+  const int poll = 8, per_graph = 2;
+  RoundLength next_round(c->st_host, nrhs);
   const bool graphs = !(c->flags & DDA_FLAG_NO_GRAPHS);
   // graph of the current kernel sequence (index into c->round_graphs, which
   // may grow while this solve runs: a precision switch captures a second one)
@@ -1398,6 +1432,7 @@ void run_solve(dda_ctx* c, int solver, int nrhs, double eps, long long max_iter,
   MixedSwitch ms(o.adapt_phase, o.adapt_tau, nrhs);
   if (o.adapt) sv.mv32 = ms.mode32;
   for (int round = 0;; round++) {
+    const int its = round == 0 ? poll : next_round.update(c->st_host, nr, poll);
     if constexpr (std::is_same<T, double>::value) {
       if (!sv.mv32 && !c->e64_tuned) {  // first FP64-convolution round of a MIXED context
         c->e64_tuned = true;
@@ -1405,7 +1440,7 @@ void run_solve(dda_ctx* c, int solver, int nrhs, double eps, long long max_iter,
       }
     }
     if (!graphs || round == 0) {
-      for (int k = 0; k < poll; k++) sv.iteration(solver, nr++, b);
+      for (int k = 0; k < its; k++) sv.iteration(solver, nr++, b);
     } else {
       const int gkey = (int)sizeof(T) + (sv.mv32 ? 100 : 0);  // kernel sequences differ per variant
       int gi = find_graph(gkey);
@@ -1414,7 +1449,7 @@ void run_solve(dda_ctx* c, int solver, int nrhs, double eps, long long max_iter,
         cudaGraph_t graph = nullptr;
         CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         try {
-          for (int k = 0; k < poll; k++) sv.iteration(solver, nr + k, b);
+          for (int k = 0; k < per_graph; k++) sv.iteration(solver, nr + k, b);
         } catch (...) {
           cudaStreamEndCapture(c->stream, &graph);
           if (graph) cudaGraphDestroy(graph);
@@ -1429,9 +1464,11 @@ void run_solve(dda_ctx* c, int solver, int nrhs, double eps, long long max_iter,
         gi = (int)c->round_graphs.size() - 1;
         c->launches = l0;
       }
-      CK(cudaGraphLaunch(c->round_graphs[gi].g, c->stream));
-      c->launches += c->round_graphs[gi].launches;
-      nr += poll;
+      for (int k = 0; k < its; k += per_graph) {
+        CK(cudaGraphLaunch(c->round_graphs[gi].g, c->stream));
+        c->launches += c->round_graphs[gi].launches;
+      }
+      nr += its;
     }
     {
       NvtxRange wait("dda round: wait for the state");
@@ -1462,7 +1499,7 @@ void run_solve(dda_ctx* c, int solver, int nrhs, double eps, long long max_iter,
       }
       const bool gap_possible = (!o.adapt || ms.it32 > 0) && near;
       if (o.check_every > 0 && nr % o.check_every == 0 && gap_possible && check_gap(c, nrhs, b.X, B, S, o)) break;
-      if (o.adapt) {
+      if (o.adapt && nr % poll == 0) {
         if (ms.update(c->st_host, nrhs, nr, poll, o.stalled)) {
           CK(cudaMemcpyAsync(c->st, c->st_host, nrhs * sizeof(KrylovState), cudaMemcpyHostToDevice, c->stream));
           bool all_done = true;

@@ -90,7 +90,7 @@ typedef struct dda_problem {
  * kernel; neither changes the results). */
 #define DDA_FLAG_NO_AUTOTUNE 8u
 /* dda_problem.flags: launch every solver iteration kernel by kernel instead of
- * replaying captured CUDA graphs of eight iterations (the results are the
+ * replaying captured CUDA graphs of two iterations (the results are the
  * same; used by tests). */
 #define DDA_FLAG_NO_GRAPHS 16u
 /* dda_problem.flags: run the fused plane kernel as two groups of half the
