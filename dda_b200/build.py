@@ -15,7 +15,7 @@ LIB = os.path.join(HERE, "libdda_b200.so")
 SOURCES = ["dda_cuda.cu", "frontend.cpp", "serve.cpp"]
 # mv_inst.cu is compiled once per (part, double, sub): the kernel-table parts,
 # those with a kernel per grid length once per range of lengths
-MV_PARTS = [(part, dbl, sub) for dbl in (0, 1) for part in (6, 0, 5, 2, 4, 3, 1)
+MV_PARTS = [(part, dbl, sub) for dbl in (0, 1) for part in (7, 6, 0, 5, 2, 4, 3, 1)
             for sub in (range(4) if part in (0, 5, 6) else (0,))]
 HEADERS = ["fft_engine.cuh", "fft_plan.cuh", "reduce.cuh", "krylov_ops.cuh", "krylov_kernels.cuh",
            "matvec_kernels.cuh", "matvec_planned.cuh", "matvec_dispatch.cuh", "dmatrix_kernels.cuh",

@@ -508,21 +508,34 @@ template <typename T> void pick_x_tile(dda_ctx* c, Engine<T>& e) {
   e.smem_x = ((size_t)g.Gx + g.nmat + (size_t)e.tl * g.pitchx) * s;
 }
 
-// Whether a grid's y/z passes run as the three kernels of matvec_pass.cuh.
-// Against the plane kernels (whole matvec, FP32, one / two right-hand sides,
-// kernels replayed from a graph): 56^3 24.8 -> 21.3 / 25.2 -> 23.8 us, 80^3
+// Whether a grid runs the compile-time planned kernels: every length with a
+// plan, or, where the flags ask for one of the other y/z paths, with the
+// lengths those have plans for.
+inline bool planned_grid(long long Gx, long long Gy, long long Gz, uint32_t flags) {
+  if (flags & DDA_FLAG_RUNTIME_PLANS) return false;
+  if (flags & (DDA_FLAG_SPLIT_YZ | DDA_FLAG_SLOT_YZ | DDA_FLAG_YZ_GROUPS2 | DDA_FLAG_YZ_GROUPS4 | DDA_FLAG_YZ_PAIR))
+    return has_tuned_plan((int)Gx) && has_tuned_plan((int)Gy) && has_tuned_plan((int)Gz);
+  return has_plan((int)Gx) && has_plan((int)Gy) && has_plan((int)Gz);
+}
+
+// Whether a grid's y/z passes run as the three kernels of matvec_pass.cuh,
+// instead of a plane kernel.  Whole matvec, one / two right-hand sides, FP32
+// unless said, kernels replayed from a graph; against the planned plane
+// kernels of the tuned lengths: 56^3 24.8 -> 21.3 / 25.2 -> 23.8 us, 80^3
 // 34.7 -> 29.1 / 57.2 -> 36.8, 128^3 79.8 -> 54.9 / 148 -> 91, 200^3 472 -> 214
-// / 876 -> 420; FP64 80^3 55.3 -> 39.2 / 97.6 -> 58.0.  Against the
-// runtime-planned plane kernel, from 10^3 (22.2 -> 14.1) to 50^3 (52.1 ->
-// 20.3).  Up to 48 x 48 planes the planned plane kernel is one launch of 5 to
-// 9 us, and two launches more cost what the passes gain: 32^3 15.0 -> 17.5 us
-// replayed, 48^3 20.7 -> 19.5 replayed but 11.7 -> 13.4 launched one by one.
+// / 876 -> 420; FP64 80^3 55.3 -> 39.2 / 97.6 -> 58.0; against the
+// runtime-planned one, 50^3 52.1 -> 20.3.  Small planes are one small CTA of
+// k_yz_p each, and two launches more cost what the passes gain: replayed,
+// passes and plane kernel 10^3 14.1 and 11.9, 30^3 17.3 and 16.1, 42^3 19.3 and
+// 20.2 (FP64 22.0 and 24.4); launched one by one 24.6 and 18.5, 25.7 and 20.6,
+// 26.8 and 24.7.  48 x 48 (tuned): 19.5 and 20.7 replayed, 13.4 and 11.7 with
+// the launches of several contexts.
 inline bool pass_grid(long long Gx, long long Gy, long long Gz, uint32_t flags) {
   if (flags & (DDA_FLAG_SPLIT_YZ | DDA_FLAG_SLOT_YZ | DDA_FLAG_RUNTIME_PLANS | DDA_FLAG_YZ_GROUPS2 |
                DDA_FLAG_YZ_GROUPS4 | DDA_FLAG_YZ_PAIR))
     return false;
   if (!has_plan((int)Gx) || !has_plan((int)Gy) || !has_plan((int)Gz)) return false;
-  return !(has_tuned_plan((int)Gx) && Gy == Gz && (Gy == 32 || Gy == 48));
+  return !(small_length((int)Gy) && small_length((int)Gz)) && !(Gy == 48 && Gz == 48);
 }
 
 // Work buffer of the y/z passes: all planes of all right-hand sides, or as
@@ -763,7 +776,7 @@ int launch_yz(dda_ctx* c, int nrhs, cudaStream_t s, KrylovState* st, int skipmv)
     CK(cudaLaunchKernelEx(&cfg, f, e.xhat, (const typename C2<T>::t*)e.dc, g, e.yz, pz, py, (const KrylovState*)st,
                           skipmv));
   } else if (e.fused) {
-    fused_yz<T>(e, e.yz_groups)<<<dim3(g.Gx, nrhs), kNtYz, e.smem_yz, s>>>(e.xhat, e.dc, g, e.yz, pz, py, st,
+    fused_yz<T>(e, e.yz_groups)<<<dim3(g.Gx, nrhs), e.k.yz_threads ? e.k.yz_threads : kNtYz, e.smem_yz, s>>>(e.xhat, e.dc, g, e.yz, pz, py, st,
                                                                            skipmv);
   } else if (e.slot_path) {
     cudaLaunchConfig_t cfg = {};
@@ -1729,9 +1742,7 @@ int dda_create(const dda_problem* p, int precision, dda_ctx** out) {
     c->px.create(g.Gx);
     c->py.create(g.Gy);
     c->pz.create(g.Gz);
-    c->planned = pass_grid(g.Gx, g.Gy, g.Gz, c->flags) ||
-                 (has_tuned_plan(g.Gx) && has_tuned_plan(g.Gy) && has_tuned_plan(g.Gz) &&
-                  !(c->flags & DDA_FLAG_RUNTIME_PLANS));
+    c->planned = planned_grid(g.Gx, g.Gy, g.Gz, c->flags);
     c->mx.create(g.Gx, c->planned ? plan_radices(g.Gx) : std::vector<int>());
     c->my.create(g.Gy, c->planned ? plan_radices(g.Gy) : std::vector<int>());
     c->mz.create(g.Gz, c->planned ? plan_radices(g.Gz) : std::vector<int>());
@@ -2249,8 +2260,7 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
   (void)bx;
   const long long nv = p->nv, nvs = (nv + 15) / 16 * 16, nl = by * bz, R = p->max_rhs;
   const long long nmat = std::max<uint32_t>(1, p->nmat);
-  const bool planned = has_tuned_plan((int)Gx) && has_tuned_plan((int)Gy) && has_tuned_plan((int)Gz) &&
-                       !(p->flags & DDA_FLAG_RUNTIME_PLANS);
+  const bool planned = planned_grid(Gx, Gy, Gz, p->flags);
   long long bytes = 4 * (nl + 1) + 9 * nv;                    // line offsets, dipoles, permutation, materials
   bytes += 6 * (Gx + Gy + Gz) * (8 + 16 + 4 + 4);              // plans
   bytes += 4 * (Gx + Gy + Gz) * (8 + 16);                      // their stage twiddles
@@ -2266,7 +2276,7 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
 #define C(N) fused_len = fused_len || Gy == N;
     DDA_FUSED_LENGTHS(C)
 #undef C
-    const bool has_yz = !planned || (Gy == Gz && fused_len);
+    const bool has_yz = !planned || (Gy == Gz && fused_len) || (small_length((int)Gy) && small_length((int)Gz));
     if (pass_grid(Gx, Gy, Gz, p->flags))
       e += (long long)pass_buffer_bytes(Gx, Gz, by, (int)R, (size_t)s);
     else if (!(has_yz && smem_yz <= (long long)kSmemMax) || (p->flags & (DDA_FLAG_SPLIT_YZ | DDA_FLAG_SLOT_YZ)))

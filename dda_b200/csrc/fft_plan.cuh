@@ -239,8 +239,8 @@ __device__ __forceinline__ void stage_twiddles0(int off, const FftPlanDev& pl) {
   }
 }
 
-// butterfly<P, 0, INV> with the twiddles of stage_twiddles0.
-template <typename P, bool INV, typename T2>
+// butterfly<P, 0, INV, T2, NZ> with the twiddles of stage_twiddles0.
+template <typename P, bool INV, typename T2, int NZ = P::r[0]>
 __device__ __forceinline__ void butterfly0(T2* v, int j, const T2* t0) {
   constexpr int R = P::r[0];
   constexpr int S0 = P::N / R;
@@ -256,7 +256,7 @@ __device__ __forceinline__ void butterfly0(T2* v, int j, const T2* t0) {
     }
     DftN<R, INV, T2>::run(v);
   } else {
-    DftN<R, INV, T2>::run(v);
+    DftN<R, INV, T2, NZ>::run(v);
     if (j) {
 #pragma unroll
       for (int m = 1; m < R; m++) v[m] = cmul(v[m], t0[(m - 1) * S0 + j]);

@@ -35,6 +35,7 @@ template <typename T> struct MvKernels {
   XfwdF<double2> xfwd_m = nullptr, xfwd_m_pre = nullptr;
   XinvF<double2> xinv_m = nullptr;
   YzFn yz = nullptr;        // fused plane kernel (nullptr: none for this shape)
+  int yz_threads = 0;       // its threads, 0: NtYz
   YzFn yz2 = nullptr;       // the same kernel run as two groups of half the CTA
   YzFn yz4 = nullptr;       // ... and as four groups of a quarter
   YzFn pair[3] = {};        // a plane per cluster of two CTAs (k_yz_pair), 1 / 2 / 4 groups
@@ -75,6 +76,41 @@ typename MvKernels<T>::YzFn fused_kernel(bool half) {
     if (half) return k_yz_p<T, NTYZ, P, P, true, GR>;
   }
   return k_yz_p<T, NTYZ, P, P, false, GR>;
+}
+
+inline bool small_length(int n) {
+  switch (n) {
+#define C(N) case N:
+    DDA_SMALL_LENGTHS(C)
+#undef C
+    return true;
+    default: return false;
+  }
+}
+
+// Plane kernel of a small plane, y length gy, z length N: the runtime-planned
+// k_yz took 21.9 us of a matvec at 10^3 (now 11.9), 34.4 at 30^3 (16.1), 44.7 at
+// 42^3 (20.2), FP32, one right-hand side.
+constexpr int kNtSmall = 256;
+template <typename T, int N>
+void small_plane(MvKernels<T>& k, int gy) {
+  switch (gy) {
+#define C(M) \
+  case M: k.yz = k_yz_p<T, kNtSmall, typename PlanFor<N>::type, typename PlanFor<M>::type>; break;
+    DDA_SMALL_LENGTHS(C)
+#undef C
+    default: return;
+  }
+  k.yz_threads = kNtSmall;
+}
+template <typename T>
+void planned_small(MvKernels<T>& k, int gy, int gz) {
+  switch (gz) {
+#define CZ(N) case N: small_plane<T, N>(k, gy); break;
+    DDA_SMALL_LENGTHS_Z(CZ)
+#undef CZ
+    default: break;
+  }
 }
 
 // Two-CTA plane kernel for y = z = N (needs an even first radix).
@@ -244,6 +280,8 @@ void mv_part_slot(MvKernels<float>& k, int gy, int gz, int by, int bz);
 void mv_part_slot(MvKernels<double>& k, int gy, int gz, int by, int bz);
 void mv_part_pair(MvKernels<float>& k, int gy, int gz, int by, int bz);
 void mv_part_pair(MvKernels<double>& k, int gy, int gz, int by, int bz);
+void mv_part_small(MvKernels<float>& k, int gy, int gz);
+void mv_part_small(MvKernels<double>& k, int gy, int gz);
 template <int S> void mv_part_pass(MvKernels<float>& k, int gy, int gz);
 template <int S> void mv_part_pass(MvKernels<double>& k, int gy, int gz);
 
@@ -262,6 +300,7 @@ MvKernels<T> select_kernels(bool planned, int gx, int gy, int gz, int by, int bz
   mv_part_xm<0>(k, gx); mv_part_xm<1>(k, gx); mv_part_xm<2>(k, gx); mv_part_xm<3>(k, gx);
   mv_part_split(k, gy, gz, false);
   mv_part_fused(k, gy, gz, by, bz);
+  if (!k.yz) mv_part_small(k, gy, gz);
   mv_part_pair(k, gy, gz, by, bz);
   mv_part_slot(k, gy, gz, by, bz);
   mv_part_pass<0>(k, gy, gz); mv_part_pass<1>(k, gy, gz); mv_part_pass<2>(k, gy, gz); mv_part_pass<3>(k, gy, gz);

@@ -28,6 +28,13 @@ namespace dda {
   X(240) X(256) X(288) X(320) X(384) X(512)
 #define DDA_FUSED_LENGTHS(X) X(32) X(48) X(56) X(64) X(80) X(96) X(100) X(112) X(120) X(128)
 
+// Lengths whose planes, in any combination, take k_yz_p as one small CTA
+// (twice: the preprocessor does not expand a macro within itself).
+#define DDA_SMALL_LENGTHS(X) \
+  X(8) X(10) X(12) X(14) X(16) X(18) X(20) X(24) X(28) X(30) X(32) X(36) X(40) X(42)
+#define DDA_SMALL_LENGTHS_Z(X) \
+  X(8) X(10) X(12) X(14) X(16) X(18) X(20) X(24) X(28) X(30) X(32) X(36) X(40) X(42)
+
 // Lengths with compile-time plans for the x passes and for the y/z passes of
 // matvec_pass.cuh, axis by axis: every even 2,3,5,7-smooth length from 8 to 512,
 // all that the reference's grid rule gives there, in four parts that compile
@@ -138,17 +145,17 @@ inline std::vector<int> plan_radices(int n) {
 
 
 // ---- z stage 0 fused with the plane read / write (whole CTA) -------------
-// HALF: the box is half the grid along the transformed axis (bz = Gz / 2,
-// first radix even), so inputs z = j + m S0 are zero exactly for m >= R / 2
-// and the inverse keeps exactly the outputs m < R / 2: with that known at
-// compile time the zero operands and the unused outputs fold away.
+// The grid is at least twice the box: inputs z = j + m S0 with m >= (R + 1) / 2
+// are zero padding and the inverse's outputs there are dropped, which folds
+// away.  HALF: the box is half the grid along the transformed axis (bz =
+// Gz / 2, first radix even), so every other input and output is inside it.
 // Columns [l0, l0 + lw) of the W = 3 by columns, by the G threads of a group
 // (tid in [0, G), barrier `bar`: 0 = the whole CTA).
 template <typename T, int G, typename PZ, bool HALF = false>
 __device__ __forceinline__ void zp_first(const typename C2<T>::t* __restrict__ plane, int soff, int q,
                                          int by, int bz, int twz, int tid, int l0, int lw, int bar) {
   typedef typename C2<T>::t T2;
-  constexpr int R = PZ::r[0], S0 = PZ::N / R;
+  constexpr int R = PZ::r[0], S0 = PZ::N / R, NZ = (R + 1) / 2;
   T2* sm = smem_at<T>(0);
   const int nb = by * bz;
   for (int b = tid; b < lw * S0; b += G) {
@@ -156,11 +163,11 @@ __device__ __forceinline__ void zp_first(const typename C2<T>::t* __restrict__ p
     const int c = l / by, y = l - c * by;
     T2 v[R];
 #pragma unroll
-    for (int m = 0; m < R; m++) {
+    for (int m = 0; m < NZ; m++) {
       const int z = j + m * S0;
-      v[m] = (HALF ? m < R / 2 : z < bz) ? plane[c * nb + z * by + y] : czero<T2>();
+      v[m] = HALF || z < bz ? plane[c * nb + z * by + y] : czero<T2>();
     }
-    butterfly<PZ, 0, false>(v, j, sm + twz);
+    butterfly<PZ, 0, false, T2, NZ>(v, j, sm + twz);
 #pragma unroll
     for (int m = 0; m < R; m++) sm[soff + (j + m * S0) * q + l] = v[m];
   }
@@ -171,7 +178,7 @@ template <typename T, int G, typename PZ, bool HALF = false>
 __device__ __forceinline__ void zp_last(typename C2<T>::t* __restrict__ plane, int soff, int q, int by,
                                         int bz, int twz, int tid, int l0, int lw) {
   typedef typename C2<T>::t T2;
-  constexpr int R = PZ::r[0], S0 = PZ::N / R;
+  constexpr int R = PZ::r[0], S0 = PZ::N / R, NZ = (R + 1) / 2;
   T2* sm = smem_at<T>(0);
   const int nb = by * bz;
   for (int b = tid; b < lw * S0; b += G) {
@@ -182,9 +189,9 @@ __device__ __forceinline__ void zp_last(typename C2<T>::t* __restrict__ plane, i
     for (int m = 0; m < R; m++) v[m] = sm[soff + (j + m * S0) * q + l];
     butterfly<PZ, 0, true>(v, j, sm + twz);
 #pragma unroll
-    for (int m = 0; m < R; m++) {
+    for (int m = 0; m < NZ; m++) {
       const int z = j + m * S0;
-      if (HALF ? m < R / 2 : z < bz) plane[c * nb + z * by + y] = v[m];
+      if (HALF || z < bz) plane[c * nb + z * by + y] = v[m];
     }
   }
 }
@@ -275,7 +282,7 @@ template <typename T, int G, typename PY, bool INV, bool HALF = false>
 __device__ __forceinline__ void rows_stage0(typename C2<T>::t* S, int kz0, int nr, int q, int by, int ro,
                                             int py, int twy, int tid, int bar) {
   typedef typename C2<T>::t T2;
-  constexpr int R = PY::r[0], S0 = PY::N / R;
+  constexpr int R = PY::r[0], S0 = PY::N / R, NZ = (R + 1) / 2;
   T2* sm = smem_at<T>(0);
   const int total = nr * 3 * S0;
   for (int it = tid; it < total; it += G) {
@@ -286,11 +293,11 @@ __device__ __forceinline__ void rows_stage0(typename C2<T>::t* S, int kz0, int n
     T2 v[R];
     if (!INV) {
 #pragma unroll
-      for (int m = 0; m < R; m++) {
+      for (int m = 0; m < NZ; m++) {
         const int yy = j + m * S0;
-        v[m] = (HALF ? m < R / 2 : yy < by) ? S[srow + yy] : czero<T2>();
+        v[m] = HALF || yy < by ? S[srow + yy] : czero<T2>();
       }
-      butterfly0<PY, false>(v, j, sm + twy);
+      butterfly0<PY, false, T2, NZ>(v, j, sm + twy);
 #pragma unroll
       for (int m = 0; m < R; m++) sm[rb + j + m * S0] = v[m];
     } else {
@@ -298,9 +305,9 @@ __device__ __forceinline__ void rows_stage0(typename C2<T>::t* S, int kz0, int n
       for (int m = 0; m < R; m++) v[m] = sm[rb + j + m * S0];
       butterfly0<PY, true>(v, j, sm + twy);
 #pragma unroll
-      for (int m = 0; m < R; m++) {
+      for (int m = 0; m < NZ; m++) {
         const int yy = j + m * S0;
-        if (HALF ? m < R / 2 : yy < by) S[srow + yy] = v[m];
+        if (HALF || yy < by) S[srow + yy] = v[m];
       }
     }
   }

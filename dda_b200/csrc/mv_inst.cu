@@ -1,17 +1,17 @@
 // mv_inst.cu -- one part of the matvec kernel tables (matvec_dispatch.cuh),
 // compiled once per part and precision:
-//   nvcc -DDDA_MV_PART=<0..6> -DDDA_MV_DOUBLE=<0|1> -DDDA_MV_SUB=<0..3> -c mv_inst.cu
+//   nvcc -DDDA_MV_PART=<0..7> -DDDA_MV_DOUBLE=<0|1> -DDDA_MV_SUB=<0..3> -c mv_inst.cu
 // (DDA_MV_SUB: the lengths of parts 0, 5 and 6, DDA_PASS_LENGTHS_<n>)
 // Part 0: x passes; 1: split path and runtime-planned kernels; 2: fused
 // plane kernels; 3: cluster plane kernels; 4: two-CTA plane kernels; 5: x
 // passes of FP32 engines over FP64 vectors; 6: y/z passes through the work
-// buffer.  The parts hold the several
+// buffer; 7: plane kernels of small planes.  The parts hold the several
 // hundred compile-time plan instantiations and build in parallel.
 #include "kernel_shapes.cuh"
 #include "matvec_dispatch.cuh"
 
 #if !defined(DDA_MV_PART) || !defined(DDA_MV_DOUBLE)
-#error "build with -DDDA_MV_PART=<0..6> -DDDA_MV_DOUBLE=<0|1>"
+#error "build with -DDDA_MV_PART=<0..7> -DDDA_MV_DOUBLE=<0|1>"
 #endif
 
 namespace dda {
@@ -48,6 +48,8 @@ template void mv_part_xm<DDA_MV_SUB>(MvKernels<MvT>&, int);
 #elif DDA_MV_PART == 6
 template <int S> void mv_part_pass(MvKernels<MvT>& k, int gy, int gz) { planned_pass<MvT, S>(k, gy, gz); }
 template void mv_part_pass<DDA_MV_SUB>(MvKernels<MvT>&, int, int);
+#elif DDA_MV_PART == 7
+void mv_part_small(MvKernels<MvT>& k, int gy, int gz) { planned_small<MvT>(k, gy, gz); }
 #endif
 
 }  // namespace dda

@@ -1,5 +1,5 @@
-"""The y/z passes as three kernels (matvec_pass.cuh) and the planned x passes
-against the oracle, at FP64 1e-12 and FP32 2e-6 relative in the 2-norm as for
+"""The y/z passes as three kernels (matvec_pass.cuh), the plane kernel of small
+planes and the planned x passes against the oracle, at FP64 1e-12 and FP32 2e-6 relative in the 2-norm as for
 the other matvec paths: two- and three-stage plans on every axis, odd and even
 first radices, last radices 2 to 8, boxes of half the grid and of less, one
 right-hand side (W = 1), a pair, and a pair with an idle lane."""
@@ -20,6 +20,8 @@ BOXES = {
     (140, 6, 5): (280, 12, 10),        # three stages along x
     (6, 125, 8): (12, 250, 16),        # ... y
     (5, 6, 150): (10, 12, 300),        # ... z
+    (20, 21, 21): (40, 42, 42),        # the largest small plane
+    (5, 21, 22): (10, 42, 48),     # ... and one beyond it
     (8, 110, 128): (16, 224, 256),
     (4, 63, 126): (8, 126, 252),
 }
@@ -35,7 +37,7 @@ def test_passes_match_oracle(box, prec, tol):
     pos = np.stack([x[keep], y[keep], z[keep]], axis=1).astype(np.uint32)
     mat = (rng.random(len(pos)) < 0.4).astype(np.uint8)
     pr = Pair("arrays", (pos, mat, "0.1um"), [1.5 + 0.1j, 1.3 + 0.02j], "1.1um", prec, max_rhs=3)
-    assert pr.p.grid == BOXES[box] and pr.mv.passes
+    assert pr.p.grid == BOXES[box] and pr.mv.passes == (max(pr.p.grid[1:]) > 42)
     xs = [pr.rand_vec(40 + r) for r in range(3)]
     want = []
     for r, pol in enumerate((1, 2, 1)):
