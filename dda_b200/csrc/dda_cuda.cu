@@ -657,7 +657,7 @@ template <typename T> void setup_engine(dda_ctx* c) {
   }
   if (e.pass) {
     auto attrs = [&](const auto& k) {
-      if (!k.rows) return;
+      if (!k.rows || !k.zfwd) return;
       attr((const void*)k.zfwd, k.smem_z);
       attr((const void*)k.zinv, k.smem_z);
       attr((const void*)k.rows, k.smem_rows);
@@ -756,7 +756,8 @@ int launch_yz(dda_ctx* c, int nrhs, cudaStream_t s, KrylovState* st, int skipmv)
   const FftPlanDev py = c->my.dev<T>(), pz = c->mz.dev<T>();
   if (e.pass) {
     if constexpr (sizeof(T) == 4)
-      if (nrhs > 1) return launch_pass<T, 2>(c, e.k.pass2, nrhs, s, st, skipmv);
+      if (nrhs > 1 && e.k.pass2.zfwd && e.k.pass2.rows)
+        return launch_pass<T, 2>(c, e.k.pass2, nrhs, s, st, skipmv);
     return launch_pass<T, 1>(c, e.k.pass1, nrhs, s, st, skipmv);
   }
   if (e.fused && e.yz_pair) {
@@ -2384,11 +2385,14 @@ void far_field_many(dda_ctx* c, int nrhs, const double* ddirs, long long ndir, d
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
   const int zr = (nrhs + NR - 1) / NR, nd = 32 * DL;
   // directions per launch and splits of the lines: about eight waves of CTAs,
-  // at least two lines per warp, within the room
+  // within the room; at least two lines per warp, or eight where the
+  // directions alone fill half the SMs, as each split computes its x phases
+  // again (21 x 12 x 14, 2 978 directions: ten splits 220 us, two 177)
   const long long fit = std::max<long long>(1, (long long)(part_bytes / row));
   const long long ctas = (std::min(ndir, fit) + nd - 1) / nd * zr;
   long long splits = (16LL / DL * nsm + ctas - 1) / ctas;
-  splits = std::max<long long>(1, std::min<long long>({splits, 64, g.nlines / (2 * (kNtFf / 32)), fit / nd}));
+  const int lines = 2 * ctas >= nsm ? 8 : 2;
+  splits = std::max<long long>(1, std::min<long long>({splits, 64, g.nlines / (lines * (kNtFf / 32)), fit / nd}));
   const long long block = std::min<long long>(ndir, fit / splits);
   for (long long d0 = 0; d0 < ndir; d0 += block) {
     const int n = (int)std::min(block, ndir - d0);

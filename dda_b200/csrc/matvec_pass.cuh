@@ -198,7 +198,10 @@ template <typename V, typename P> struct ZTile {
 
 // Rows per CTA of k_rows (of the four mirrored ones) and its threads: all four
 // while they take at most 48 KB, so that four to seven CTAs share an SM (160:
-// four rows 79.5 us, two 90.4; 512: one row 974 us, four 2 400).
+// four rows 79.5 us, two 90.4; 512: one row 974 us, four 2 400).  Registers per
+// thread: as many as leave the most warps without spills that cost more (FP64,
+// 16 x 8: 128 registers 482 us, 160 438; 20 x 5: 89 and 95; P2, 16 x 8: 383 and
+// 407; FP32, 32 x 8: 80 registers 296 us, 96 286).
 template <typename V, typename P> struct RTile {
   enum : int {
     LINE = 3 * RowPad<P>::pitch(sizeof(V)) * (int)sizeof(V),
@@ -206,7 +209,10 @@ template <typename V, typename P> struct RTile {
     IT0 = RQ * 3 * (P::N / P::r[0]),
     IT1 = RQ * (P::N / P::r[P::K - 1]),
     NT = pass_threads(P::K == 2 ? IT1 : IT0, 128),
-    REGS = sizeof(V) == 16 ? 128 : 80,
+    REGS = std::is_same<V, double2>::value ? (P::K == 2 && P::r[P::K - 1] == 8 ? 160 : 128)
+           : sizeof(V) == 16               ? 128
+           : P::r[0] >= 28                 ? 96
+                                           : 80,
     CTAS = pass_ctas(NT, REGS)
   };
 };
@@ -498,21 +504,32 @@ template <typename T, int W> struct PassKernels {
   size_t smem_z = 0, smem_rows = 0;
 };
 
+// Pairs of right-hand sides pay while a first butterfly of them fits the
+// registers (240 = 30 x 8: z forward, z inverse and rows 118, 117 and 310 us in
+// pairs, 103, 121 and 263 one by one).
+template <int W, typename P> constexpr bool pass_width() { return W == 1 || P::r[0] < 30; }
+
 template <typename T, int W, typename P> void pass_z(PassKernels<T, W>& k) {
-  typedef ZTile<typename PassV<T, W>::t, P> Z;
-  k.zfwd = k_zfwd<T, W, P>;
-  k.zinv = k_zinv<T, W, P>;
-  k.ztc = Z::TC;
-  k.ntf = Z::NTF;
-  k.nti = Z::NTI;
-  k.smem_z = (size_t)P::N * Z::SEG + StageTw<P>::count() * sizeof(typename C2<T>::t);
+  if constexpr (!pass_width<W, P>()) return;
+  else {
+    typedef ZTile<typename PassV<T, W>::t, P> Z;
+    k.zfwd = k_zfwd<T, W, P>;
+    k.zinv = k_zinv<T, W, P>;
+    k.ztc = Z::TC;
+    k.ntf = Z::NTF;
+    k.nti = Z::NTI;
+    k.smem_z = (size_t)P::N * Z::SEG + StageTw<P>::count() * sizeof(typename C2<T>::t);
+  }
 }
 template <typename T, int W, typename P> void pass_y(PassKernels<T, W>& k) {
-  typedef RTile<typename PassV<T, W>::t, P> R;
-  k.rows = k_rows<T, W, P>;
-  k.ntr = R::NT;
-  k.rows_per = 4 / R::RQ;
-  k.smem_rows = rows_smem<T, W, P>();
+  if constexpr (!pass_width<W, P>()) return;
+  else {
+    typedef RTile<typename PassV<T, W>::t, P> R;
+    k.rows = k_rows<T, W, P>;
+    k.ntr = R::NT;
+    k.rows_per = 4 / R::RQ;
+    k.smem_rows = rows_smem<T, W, P>();
+  }
 }
 
 }  // namespace dda

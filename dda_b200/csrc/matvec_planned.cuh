@@ -53,8 +53,9 @@ namespace dda {
   DDA_PASS_LENGTHS_0(X) DDA_PASS_LENGTHS_1(X) DDA_PASS_LENGTHS_2(X) DDA_PASS_LENGTHS_3(X)
 
 // Plans: a large first radix and a last radix of at most 8, so the fused last
-// y stage holds 3 x R_last complex values per thread; two stages up to 240
-// (in the row kernel a stage more costs half as much again), three beyond.
+// y stage holds 3 x R_last complex values per thread; two stages up to 256
+// but for 250 and 252, three beyond (in the row kernel a stage more costs half
+// as much again: 256 as 8 x 4 x 8 428 us, as 32 x 8 286).
 template <int N> struct PlanFor { typedef void type; };
 template <> struct PlanFor<8> { typedef Plan<2, 4> type; };
 template <> struct PlanFor<10> { typedef Plan<2, 5> type; };
@@ -105,7 +106,7 @@ template <> struct PlanFor<224> { typedef Plan<28, 8> type; };
 template <> struct PlanFor<240> { typedef Plan<30, 8> type; };
 template <> struct PlanFor<250> { typedef Plan<10, 5, 5> type; };
 template <> struct PlanFor<252> { typedef Plan<12, 3, 7> type; };
-template <> struct PlanFor<256> { typedef Plan<8, 4, 8> type; };
+template <> struct PlanFor<256> { typedef Plan<32, 8> type; };
 template <> struct PlanFor<270> { typedef Plan<9, 6, 5> type; };
 template <> struct PlanFor<280> { typedef Plan<10, 4, 7> type; };
 template <> struct PlanFor<288> { typedef Plan<6, 6, 8> type; };
