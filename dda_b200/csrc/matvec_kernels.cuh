@@ -66,12 +66,14 @@ __device__ __forceinline__ void load_dhat(const typename C2<T>::t* __restrict__ 
 }
 
 // y = D x for the symmetric 3x3 matrix (xx, xy, xz, yy, yz, zz)
-// (Math/SymMatrix3.hpp:86-92).
+// (Math/SymMatrix3.hpp:86-92).  The diagonal product, mostly the largest of
+// the three, is added last, so that the roundings before it are of a smaller
+// sum.
 template <typename V, typename W>
 __device__ __forceinline__ void dmul(const W d[6], V& a, V& b, V& c) {
   const V x = a, y = b, z = c;
-  a = cfma(cfma(cmul(x, d[0]), d[1], y), d[2], z);
-  b = cfma(cfma(cmul(x, d[1]), d[3], y), d[4], z);
+  a = cfma(cfma(cmul(z, d[2]), d[1], y), d[0], x);
+  b = cfma(cfma(cmul(x, d[1]), d[4], z), d[3], y);
   c = cfma(cfma(cmul(x, d[2]), d[4], y), d[5], z);
 }
 
@@ -332,7 +334,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 3) k_xfwd(const A2* _
         }
         T2 x = cvt<T2>(v[u]);
         if (conj) x.y = -x.y;
-        sm[o[u] + (d[u] & 0xffffu)] = cmul(x, scc[d[u] >> 16]);
+        sm[o[u] + (d[u] & 0xffffu)] = cmul_re(x, scc[d[u] >> 16]);
       }
   }
   if (PRE && blockIdx.x == 0)
@@ -446,10 +448,10 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 3) k_xinv(const A2* _
         if constexpr (std::is_same<A2, T2>::value) {
           T2 av = a0[u];
           if (conj) av.y = -av.y;
-          y = cadd(cmul(x, scc[d[u] >> 16]), av);
+          y = cadd(cmul_re(x, scc[d[u] >> 16]), av);
           if (conj) y.y = -y.y;
         } else {
-          T2 cv = cmul(x, scc[d[u] >> 16]);
+          T2 cv = cmul_re(x, scc[d[u] >> 16]);
           if (conj) cv.y = -cv.y;
           y = a0[u];
           y.x += cv.x;

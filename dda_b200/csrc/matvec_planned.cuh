@@ -55,7 +55,11 @@ namespace dda {
 // Plans: a large first radix and a last radix of at most 8, so the fused last
 // y stage holds 3 x R_last complex values per thread; two stages up to 256
 // but for 250 and 252, three beyond (in the row kernel a stage more costs half
-// as much again: 256 as 8 x 4 x 8 428 us, as 32 x 8 286).
+// as much again: 256 as 8 x 4 x 8 428 us, as 32 x 8 286).  Where several do,
+// the radices with the smaller FP32 error of a product against 64 bits: 512^3 as
+// 8 x 8 x 8 1.13e-7 (8.3 ms), as 16 x 4 x 8 1.29e-7 (8.1 ms); an axis of 288 as
+// 12 x 3 x 8 4.7 % less than as 6 x 6 x 8, one of 480 as 12 x 5 x 8 4.8 % less
+// than as 16 x 6 x 5.
 template <int N> struct PlanFor { typedef void type; };
 template <> struct PlanFor<8> { typedef Plan<2, 4> type; };
 template <> struct PlanFor<10> { typedef Plan<2, 5> type; };
@@ -109,7 +113,7 @@ template <> struct PlanFor<252> { typedef Plan<12, 3, 7> type; };
 template <> struct PlanFor<256> { typedef Plan<32, 8> type; };
 template <> struct PlanFor<270> { typedef Plan<9, 6, 5> type; };
 template <> struct PlanFor<280> { typedef Plan<10, 4, 7> type; };
-template <> struct PlanFor<288> { typedef Plan<6, 6, 8> type; };
+template <> struct PlanFor<288> { typedef Plan<12, 3, 8> type; };
 template <> struct PlanFor<294> { typedef Plan<14, 3, 7> type; };
 template <> struct PlanFor<300> { typedef Plan<12, 5, 5> type; };
 template <> struct PlanFor<320> { typedef Plan<5, 8, 8> type; };
@@ -125,12 +129,12 @@ template <> struct PlanFor<420> { typedef Plan<12, 5, 7> type; };
 template <> struct PlanFor<432> { typedef Plan<12, 6, 6> type; };
 template <> struct PlanFor<448> { typedef Plan<16, 4, 7> type; };
 template <> struct PlanFor<450> { typedef Plan<15, 6, 5> type; };
-template <> struct PlanFor<480> { typedef Plan<16, 6, 5> type; };
+template <> struct PlanFor<480> { typedef Plan<12, 5, 8> type; };
 template <> struct PlanFor<486> { typedef Plan<9, 9, 6> type; };
 template <> struct PlanFor<490> { typedef Plan<14, 5, 7> type; };
 template <> struct PlanFor<500> { typedef Plan<20, 5, 5> type; };
 template <> struct PlanFor<504> { typedef Plan<12, 6, 7> type; };
-template <> struct PlanFor<512> { typedef Plan<16, 4, 8> type; };
+template <> struct PlanFor<512> { typedef Plan<8, 8, 8> type; };
 
 // Radices of the compile-time plan for n (host side), empty when there is none.
 inline std::vector<int> plan_radices(int n) {
