@@ -2449,38 +2449,54 @@ void far_field_t(dda_ctx* c, int nrhs, const double* pol, long long ndir, const 
 // (24*ndir bytes, rounded up to 256), fields after them (48*ndir*nrhs
 // bytes).  Nothing in it needs to start at zero: each call writes every
 // byte it later reads.  One array per device, shared by every context on
-// that device, so calls that overlap in time race on it.
+// that device: a call holds the device's lock from its first write to it
+// until its work is done.
 constexpr size_t kFfScratchBytes = size_t(1) << 20;
 static __device__ __align__(256) unsigned char g_ff_scratch[kFfScratchBytes];
 
 constexpr int kFfMaxDevices = 64;
-std::mutex g_ff_scratch_mu;
-unsigned char* g_ff_scratch_ptr[kFfMaxDevices];
+struct FfScratch {
+  std::mutex mu;
+  unsigned char* ptr = nullptr;  // on the device, looked up by its first call
+};
+FfScratch g_ff_scratches[kFfMaxDevices];
 
 size_t ff_noalloc_bytes(long long ndir, int nrhs) {
   return (((size_t)ndir * 3 * sizeof(double) + 255) & ~(size_t)255) + (size_t)ndir * nrhs * 3 * sizeof(double2);
 }
 
-// Address of the scratch on `device`, which must be the current device.
-// Looked up once per device, on the first call there.
-unsigned char* ff_scratch(int device) {
-  if (device < 0 || device >= kFfMaxDevices)
-    throw DdaError(DDA_ERR_UNSUPPORTED, "device ordinal beyond the no-allocation far-field table");
-  std::lock_guard<std::mutex> lock(g_ff_scratch_mu);
-  if (!g_ff_scratch_ptr[device]) {
-    void* ptr = nullptr;
-    const cudaError_t rc = cudaGetSymbolAddress((void**)&ptr, g_ff_scratch);
-    if (rc != cudaSuccess || !ptr)
+// The scratch of a context's device, locked for the life of this object.
+// The stream is waited for before the lock is given back, also when an error
+// leaves the call early.
+class FfScratchLock {
+ public:
+  explicit FfScratchLock(dda_ctx* c) : stream_(c->stream), lock_(scratch(c->device).mu) {
+    unsigned char*& ptr = scratch(c->device).ptr;
+    if (ptr) return;
+    void* p = nullptr;
+    const cudaError_t rc = cudaGetSymbolAddress(&p, g_ff_scratch);  // of the current device, the context's
+    if (rc != cudaSuccess || !p)
       throw DdaError(DDA_ERR_CUDA, std::string("cudaGetSymbolAddress of the far-field scratch: ") +
                                        cudaGetErrorString(rc));
-    g_ff_scratch_ptr[device] = static_cast<unsigned char*>(ptr);
+    ptr = static_cast<unsigned char*>(p);
   }
-  return g_ff_scratch_ptr[device];
-}
+  ~FfScratchLock() { cudaStreamSynchronize(stream_); }
+  unsigned char* ptr(const dda_ctx* c) const { return scratch(c->device).ptr; }
+
+ private:
+  static FfScratch& scratch(int device) {
+    if (device < 0 || device >= kFfMaxDevices)
+      throw DdaError(DDA_ERR_UNSUPPORTED, "device ordinal beyond the no-allocation far-field table");
+    return g_ff_scratches[device];
+  }
+  cudaStream_t stream_;
+  std::unique_lock<std::mutex> lock_;  // released after the destructor's wait
+};
 
 template <typename T>
 void far_field_noalloc_t(dda_ctx* c, int nrhs, long long ndir, const double* dirs, double* out) {
-  unsigned char* scratch = ff_scratch(c->device);
+  const FfScratchLock held(c);
+  unsigned char* scratch = held.ptr(c);
   double* ddirs = reinterpret_cast<double*>(scratch);
   double2* dout = reinterpret_cast<double2*>(scratch + ((ndir * 3 * sizeof(double) + 255) & ~(size_t)255));
   CK(cudaMemcpyAsync(ddirs, dirs, ndir * 3 * sizeof(double), cudaMemcpyHostToDevice, c->stream));

@@ -268,10 +268,10 @@ int dda_far_field(dda_ctx* ctx, int nrhs, const double* pol, int64_t ndir, const
  *
  * For callers that must not allocate device memory while they evaluate far
  * fields: a serving loop that keeps solves of other contexts in flight on
- * other streams of the same device (cudaFree waits for the whole device,
- * which would stall those solves), or a process that has handed the free
- * device memory to its solver contexts (dda_far_field's per-call cudaMalloc
- * then fails with DDA_ERR_OOM).
+ * other streams of the same device, or a process that has handed the free
+ * device memory to its solver contexts (a dda_far_field of more directions
+ * than the context's solver vectors hold allocates, and then fails with
+ * DDA_ERR_OOM).
  *
  * Limit: 24*ndir bytes rounded up to 256, plus 48*ndir*nrhs bytes, at most
  * 1 MiB (14,560 directions for one right-hand side, 8,736 for two); larger
@@ -284,8 +284,8 @@ int dda_far_field(dda_ctx* ctx, int nrhs, const double* pol, int64_t ndir, const
  * any other reset of that device's primary context) in the same process:
  * the kept address would no longer be valid.  Every context on
  * a device shares the one scratch array: calls that overlap in time (from
- * two host threads, on any contexts of the same device) race on it and must
- * be serialised by the caller.  Each call returns after `out` is written. */
+ * several host threads, on any contexts of the same device) run one after
+ * another.  Each call returns after `out` is written. */
 int dda_far_field_noalloc(dda_ctx* ctx, int nrhs, int64_t ndir, const double* dirs, double* out);
 
 /* Copies the D matrix out in the reference layout ([Gx][Gz][Gy][6] complex

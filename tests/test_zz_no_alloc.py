@@ -48,3 +48,28 @@ def test_noalloc_far_field_rejects_beyond_scratch():
     out = mv.far_field_noalloc(dirs[:8736], nrhs=2)  # 1,048,320 bytes
     want = mv.far_field(dirs[:1], nrhs=2)
     assert np.abs(out[-1] - want[0]).max() <= 1e-12 * np.abs(want).max()
+
+
+def test_noalloc_far_fields_of_two_threads():
+    # the contexts of a device share the scratch: calls from two threads take
+    # their turns, each with its own directions and fields
+    import threading
+    mvs = [_solved("fp64"), _solved("fp32")]
+    rng = np.random.default_rng(5)
+    dirs = [rng.normal(size=(n, 3)) for n in (3000, 8736)]
+    dirs = [d / np.linalg.norm(d, axis=1, keepdims=True) for d in dirs]
+    want = [mv.far_field(d, nrhs=2) for mv, d in zip(mvs, dirs)]
+    bad = []
+
+    def work(i):
+        for _ in range(20):
+            got = mvs[i].far_field_noalloc(dirs[i], nrhs=2)
+            if not np.abs(got - want[i]).max() <= 1e-12 * np.abs(want[i]).max():
+                bad.append(i)
+
+    t = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for x in t:
+        x.start()
+    for x in t:
+        x.join()
+    assert not bad
