@@ -31,6 +31,9 @@ class Problem(ctypes.Structure):
                 ("device", ctypes.c_int32), ("flags", ctypes.c_uint32)]
 
 FLAG_SPLIT_YZ = 1
+FLAG_RUNTIME_PLANS = 2
+FLAG_SLOT_YZ = 4
+FLAG_NO_AUTOTUNE = 8
 FLAG_YZ_GROUPS2 = 32
 FLAG_YZ_GROUPS4 = 64
 FLAG_YZ_PAIR = 128
@@ -509,12 +512,16 @@ class CudaMatVec:
         if d["yz_path"] == "fused":  # slots 1, 2: CTAs per plane and thread groups
             d["groups"] = d.pop("cluster_size")
             d["ctas_per_plane"] = d.pop("clusters")
+        elif d["yz_path"] == "passes":
+            d["rows_per_cta"] = d.pop("clusters")
+            d["columns_per_cta"] = d.pop("cluster_size")
+            d["rhs_side_by_side"] = d.pop("rows_per_batch")
         return d
 
     @property
     def passes(self):
         """True when matvecs run their y/z passes as three kernels over a work
-        buffer instead of the plane kernel that `layout` describes."""
+        buffer instead of a plane kernel."""
         return bool(lib().dda_matvec_passes(self.h))
 
     def profile(self, nrhs=1, reps=10):

@@ -436,7 +436,7 @@ template <typename T> void setup_slot(dda_ctx* c, Engine<T>& e) {
   }
   e.order = (uint32_t*)dalloc<float>(order.size() * sizeof(uint32_t));
   CK(cudaMemcpyAsync(e.order, order.data(), order.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
-  if (!e.pass) e.slots = (T2*)dalloc<T>((size_t)ncl_max * g.Gz * sg.wp * sizeof(T2));
+  e.slots = (T2*)dalloc<T>((size_t)ncl_max * g.Gz * sg.wp * sizeof(T2));
   e.sg = sg;
   e.cl = cl;
   e.ncl = ncl;
@@ -551,13 +551,13 @@ inline size_t pass_buffer_bytes(long long Gx, long long Gz, long long by, int ma
   return std::max(4 * plane, std::min(all, kPassCap));
 }
 
-// Chooses tile shapes and allocates the matvec buffers of one precision.
-template <typename T> void setup_engine(dda_ctx* c) {
+// The plane kernel of one precision, its tile shapes and buffers: the y/z
+// path of the grids whose y/z passes do not run as three kernels.
+template <typename T> void setup_plane(dda_ctx* c) {
   typedef typename C2<T>::t T2;
   Engine<T>& e = eng<T>(c);
   const MvGeom& g = c->g;
   const size_t s = sizeof(T2);
-  e.on = true;
   constexpr int NW = kNtYz / 32;
   // fused plane kernel: twiddles, slab Gz x q, row buffers 3 x (Gy+1)
   YzGeom y;
@@ -565,7 +565,6 @@ template <typename T> void setup_engine(dda_ctx* c) {
   y.py = g.Gy + 1;
   const size_t fixed = ((size_t)g.Gz + g.Gy + (size_t)g.Gz * y.q) * s;
   const size_t row = (size_t)3 * y.py * s;
-  e.k = select_kernels<T>(c->planned, g.Gx, g.Gy, g.Gz, g.by, g.bz);
   // row buffers: one per warp in the runtime-planned kernel, batches of up
   // to 32 rows in the planned one
   int nrw = c->planned ? 32 : NW;
@@ -602,9 +601,8 @@ template <typename T> void setup_engine(dda_ctx* c) {
     e.yz.nrw = nrw - nrw % forced;  // a multiple of the groups: an equal share each
     e.smem_yz = fixed + e.yz.nrw * row;
   }
-  e.pass = pass_grid(g.Gx, g.Gy, g.Gz, c->flags);
   if (!e.fused && e.k.slot && !(c->flags & DDA_FLAG_SPLIT_YZ)) setup_slot<T>(c, e);
-  if (!e.fused && !e.slot_path && !e.pass) {
+  if (!e.fused && !e.slot_path) {
     // split path: zbuf, k_yrows over NW rows per CTA, column FFTs along z
     e.yz.nrw = NW;
     e.smem_rows = ((size_t)g.Gy + (size_t)NW * 3 * y.py) * s;
@@ -635,6 +633,18 @@ template <typename T> void setup_engine(dda_ctx* c) {
       throw DdaError(DDA_ERR_UNSUPPORTED, "FFT grid too large for the shared-memory tiles");
     e.zbuf = (T2*)dalloc<T>((size_t)c->max_rhs * g.Gx * 3 * g.Gz * g.by * s);
   }
+}
+
+// Chooses tile shapes and allocates the matvec buffers of one precision.
+template <typename T> void setup_engine(dda_ctx* c) {
+  typedef typename C2<T>::t T2;
+  Engine<T>& e = eng<T>(c);
+  const MvGeom& g = c->g;
+  const size_t s = sizeof(T2);
+  e.on = true;
+  e.k = select_kernels<T>(c->planned, g.Gx, g.Gy, g.Gz, g.by, g.bz);
+  e.pass = pass_grid(g.Gx, g.Gy, g.Gz, c->flags);
+  if (!e.pass) setup_plane<T>(c);
   pick_x_tile<T>(c, e);
   if (e.smem_x > kSmemMax) throw DdaError(DDA_ERR_UNSUPPORTED, "grid x extent too large");
   // (a kernel that stays within the 48 KB every kernel may use is not looked
@@ -645,7 +655,7 @@ template <typename T> void setup_engine(dda_ctx* c) {
     CK(allow_smem(f));
   };
   for (const void* f : x_pass_kernels(e)) attr(f, e.smem_x);
-  if (e.fused && !e.pass) {  // the autotuner may take up to all of it
+  if (e.fused) {  // the autotuner may take up to all of it
     for (int gr : {1, 2, 4})
       if (fused_yz<T>(e, gr)) attr((const void*)fused_yz<T>(e, gr), kSmemMax);
     for (auto f : e.k.pair)
@@ -823,11 +833,11 @@ template <typename T> float time_yz(dda_ctx* c, int nrhs, int reps) {
   cudaEvent_t a, b;
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
-  launch_yz<T>(c, nrhs, c->stream, nullptr, 0);  // warm-up
+  c->launches += launch_yz<T>(c, nrhs, c->stream, nullptr, 0);  // warm-up
   float best = 1e30f;
   for (int r = 0; r < reps; r++) {
     CK(cudaEventRecord(a, c->stream));
-    launch_yz<T>(c, nrhs, c->stream, nullptr, 0);
+    c->launches += launch_yz<T>(c, nrhs, c->stream, nullptr, 0);
     CK(cudaEventRecord(b, c->stream));
     CK(cudaEventSynchronize(b));
     float ms = 0;
@@ -858,7 +868,7 @@ template <typename T> void apply_choice(dda_ctx* c, Engine<T>& e, const TuneChoi
 template <typename T> void autotune(dda_ctx* c) {
   Engine<T>& e = eng<T>(c);
   const MvGeom& g = c->g;
-  if (!e.on || e.pass || !(e.fused || e.slot_path)) return;
+  if (!e.on || !(e.fused || e.slot_path)) return;
   NvtxRange range(sizeof(T) == 4 ? "dda autotune fp32" : "dda autotune fp64");
   if ((long long)g.Gx * g.Gy * g.Gz < (1LL << 20)) return;  // small grids keep the defaults
   // the box changes the best batching little next to the grid, so shapes
@@ -2300,12 +2310,26 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
 
 int dda_matvec_layout(const dda_ctx* ctx, int64_t* out) {
   if (!ctx || !out) return DDA_ERR_ARG;
+  // of the passes: the kernels of whole batches, pairs of right-hand sides
+  // where the context may hold two and a pair kernel exists
+  auto pass = [&](const auto& k, int side_by_side) {
+    out[0] = 3;
+    out[1] = 4 / k.rows_per;
+    out[2] = k.ztc;
+    out[3] = side_by_side;
+    out[4] = (int64_t)k.smem_rows;
+  };
   auto fill = [&](const auto& e) {
-    out[0] = e.fused ? 0 : e.slot_path ? 1 : e.pass ? 3 : 2;
+    if (e.pass) {
+      if (ctx->max_rhs > 1 && e.k.pass2.zfwd && e.k.pass2.rows) pass(e.k.pass2, 2);
+      else pass(e.k.pass1, 1);
+      return;
+    }
+    out[0] = e.fused ? 0 : e.slot_path ? 1 : 2;
     out[1] = e.fused ? (e.yz_pair ? 2 : 1) : e.ncl;
     out[2] = e.fused ? e.yz_groups : e.cl;
     out[3] = e.slot_path ? e.sg.nrw : e.yz.nrw;
-    out[4] = (int64_t)(e.fused ? e.smem_yz : e.slot_path ? e.smem_slot : e.pass ? e.k.pass1.smem_rows : e.smem_rows);
+    out[4] = (int64_t)(e.fused ? e.smem_yz : e.slot_path ? e.smem_slot : e.smem_rows);
   };
   if (ctx->e32.on) fill(ctx->e32);
   else fill(ctx->e64);

@@ -96,7 +96,10 @@ template <typename T, int N>
 void small_plane(MvKernels<T>& k, int gy) {
   switch (gy) {
 #define C(M) \
-  case M: k.yz = k_yz_p<T, kNtSmall, typename PlanFor<N>::type, typename PlanFor<M>::type>; break;
+  case M:                                                                                              \
+    if constexpr (!(M == 32 && N == 32)) /* has the tuned kernel */                                     \
+      k.yz = k_yz_p<T, kNtSmall, typename PlanFor<N>::type, typename PlanFor<M>::type>;                \
+    break;
     DDA_SMALL_LENGTHS(C)
 #undef C
     default: return;

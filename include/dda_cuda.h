@@ -225,21 +225,24 @@ int dda_footprint(const dda_problem* prob, int precision, int64_t* resident, int
 
 /* Layout the context chose for its matvec (working precision: FP32 for
  * DDA_PREC_FP32 and DDA_PREC_MIXED, FP64 otherwise), 8 values:
- * [0] plane kernel of the grid (0 fused plane kernel, 1 cluster kernel, 2 split
- * path, 3 none: the y/z passes only, see dda_matvec_passes),
- * [1] resident clusters (cluster kernel) or CTAs per kx plane (fused
- * kernels: 1, or 2 for the two-CTA kernel), [2] CTAs per cluster (cluster kernel) or thread
- * groups per CTA (fused kernel: 1, 2 or 4), [3] rows per y batch,
- * [4] dynamic shared memory of the y/z kernel (bytes), [5] grid lines per
- * x tile, [6] compile-time FFT plans (1) or runtime plans (0),
+ * [0] y/z path (0 fused plane kernel, 1 cluster kernel, 2 split path, 3 the
+ * passes: three kernels over a work buffer),
+ * [1] resident clusters (cluster kernel), CTAs per kx plane (fused kernels:
+ * 1, or 2 for the two-CTA kernel) or rows per CTA (passes), [2] CTAs per
+ * cluster (cluster kernel), thread groups per CTA (fused kernel: 1, 2 or 4)
+ * or columns per CTA of the z kernels (passes), [3] rows per y batch, or
+ * right-hand sides side by side in a kernel (passes),
+ * [4] dynamic shared memory of the y/z kernel (passes: of the row kernel;
+ * bytes), [5] grid lines per x tile,
+ * [6] compile-time FFT plans (1) or runtime plans (0),
  * [7] device bytes the context holds.  A diagnostic for tuning and
  * benchmark reports; no counterpart in the reference. */
 int dda_matvec_layout(const dda_ctx* ctx, int64_t* out);
 
 /* 1 when the context's matvecs (working precision) run their y/z passes as
  * the three kernels z forward, y rows with the D multiply, z inverse over a
- * work buffer, 0 when they run the plane kernel that dda_matvec_layout
- * describes.  A diagnostic; no counterpart in the reference. */
+ * work buffer (dda_matvec_layout [0] = 3), 0 when they run a plane kernel.  A
+ * diagnostic; no counterpart in the reference. */
 int dda_matvec_passes(const dda_ctx* ctx);
 
 /* Times the stages of one matvec of nrhs right-hand sides with CUDA events

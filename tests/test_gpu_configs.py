@@ -60,17 +60,21 @@ def spheroid_oracle():
     return pos, mat, "%gum" % d_um, lam, op, rhs
 
 
-@pytest.mark.parametrize("prec,tol", [("fp64", FP64_TOL), ("fp32", FP32_TOL)])
-def test_spheroid_block_matvec_matches_oracle(spheroid_oracle, prec, tol):
+@pytest.mark.parametrize("prec,tol,flags,ctas", [
+    ("fp64", FP64_TOL, 0, 0), ("fp32", FP32_TOL, 0, 0),                    # the passes
+    ("fp32", FP32_TOL, dda_b200.api.FLAG_YZ_GROUPS2, 1),                   # half-padded plane kernel in one CTA
+    ("fp32", FP32_TOL, dda_b200.api.FLAG_YZ_PAIR, 2),                      # ... and in two
+    ("fp64", FP64_TOL, dda_b200.api.FLAG_YZ_PAIR, 2)])                     # (395 KB: beyond one CTA's shared memory)
+def test_spheroid_block_matvec_matches_oracle(spheroid_oracle, prec, tol, flags, ctas):
     pos, mat, gu, lam, op, rhs = spheroid_oracle
     g = dda_b200.Geometry.from_arrays(pos, mat, gu)
     p = dda_b200.DDAParams(g, [1.33 + 0.01j], lam)
     assert p.grid == (192, 128, 128) and p.box == (96, 64, 64)
-    mv = dda_b200.CudaMatVec(p, prec, max_rhs=4)
-    # FP32: the fused half-padded plane kernel in one CTA; FP64: the plane
-    # (395 KB) is beyond one CTA's shared memory, so two CTAs share it
+    mv = dda_b200.CudaMatVec(p, prec, max_rhs=4, flags=flags)
     lay = mv.layout
-    assert lay["yz_path"] == "fused" and lay["ctas_per_plane"] == (1 if prec == "fp32" else 2)
+    assert lay["yz_path"] == ("fused" if ctas else "passes")
+    if ctas:
+        assert lay["ctas_per_plane"] == ctas
     rng = np.random.default_rng(3)
     xs, want = [], []
     for r, (prop, pol) in enumerate(rhs):
@@ -115,29 +119,31 @@ def sphere512_oracle(sphere512):
 
 
 @pytest.mark.parametrize("prec,tol", [("fp64", FP64_TOL), ("fp32", FP32_TOL)])
-def test_sphere512_cluster_matvec_matches_oracle(sphere512, sphere512_oracle, prec, tol):
+def test_sphere512_matvec_matches_oracle(sphere512, sphere512_oracle, prec, tol):
     p, x = sphere512
     mv = dda_b200.CudaMatVec(p, prec)
     lay = mv.layout
-    assert lay["yz_path"] == "cluster" and lay["compile_time_plans"] == 1
+    assert lay["yz_path"] == "passes" and lay["compile_time_plans"] == 1
     mv.set_couple_constants(dda_b200.CoupleConstants(p, (0, 0, 1), 1, "ldr"))
     y = mv.apply(x)
     assert rel(y, sphere512_oracle) < tol, rel(y, sphere512_oracle)
     mv.close()
 
 
-def test_sphere512_cluster_path_equals_split_path(sphere512):
-    # the production cluster kernel and the split y/z path (tested against
-    # the oracle on small grids) on the same input, both FP64
+def test_sphere512_other_paths_equal_the_passes(sphere512):
+    # the passes (tested against the oracle above), the cluster kernel and the
+    # split y/z path on the same input, all FP64
     p, x = sphere512
     out = []
-    for flags in (0, dda_b200.api.FLAG_SPLIT_YZ):
+    for flags, path in ((0, "passes"), (dda_b200.api.FLAG_SLOT_YZ | dda_b200.api.FLAG_NO_AUTOTUNE, "cluster"),
+                        (dda_b200.api.FLAG_SPLIT_YZ, "split")):
         mv = dda_b200.CudaMatVec(p, "fp64", flags=flags)
-        assert mv.layout["yz_path"] == ("cluster" if flags == 0 else "split")
+        assert mv.layout["yz_path"] == path
         mv.set_couple_constants(dda_b200.CoupleConstants(p, (0, 0, 1), 2, "ldr"))
         out.append(mv.apply(x))
         mv.close()
-    assert rel(out[0], out[1]) < FP64_TOL
+    for other in out[1:]:
+        assert rel(out[0], other) < FP64_TOL
 
 
 # ----------------------------------------------- Jones gate, README sphere ----

@@ -4,6 +4,7 @@ FP32 2e-6, relative in the 2-norm of the result."""
 import numpy as np
 import pytest
 
+from dda_b200 import api
 from tests.pairs import Pair, aniso_arrays, scrambled_arrays, rel
 
 pytestmark = pytest.mark.gpu
@@ -82,14 +83,16 @@ def test_matvec_cluster_path_small_grids(case, prec, tol):
     assert rel(pr.mv.apply(x, conj=True), pr.op.matvec(x, conj=True)) < tol
 
 
+@pytest.mark.parametrize("flags,path", [(0, "passes"), (api.FLAG_SLOT_YZ | api.FLAG_NO_AUTOTUNE, "cluster")])
 @pytest.mark.parametrize("prec,tol", [("fp64", FP64_TOL), ("fp32", FP32_TOL)])
-def test_matvec_plane_beyond_shared_memory(prec, tol):
+def test_matvec_plane_beyond_shared_memory(prec, tol, flags, path):
     # sphere of radius 40 dipoles: grid 160^3, a kx plane (160 x 3 x 80
-    # complex) does not fit one CTA, so the default path is the cluster
-    # kernel; two right-hand sides with different couple constants
-    pr = Pair("sphere", ("2um", "0.05um"), [1.5 + 0.1j], "1.2um", prec, max_rhs=2)
+    # complex) does not fit one CTA, so the paths are the three passes (the
+    # default) and the cluster kernel; two right-hand sides with different
+    # couple constants
+    pr = Pair("sphere", ("2um", "0.05um"), [1.5 + 0.1j], "1.2um", prec, max_rhs=2, flags=flags)
     assert pr.p.grid == (160, 160, 160)
-    assert pr.mv.layout["yz_path"] == "cluster"
+    assert pr.mv.layout["yz_path"] == path
     xs = [pr.rand_vec(31), pr.rand_vec(32)]
     want = []
     for r, pol in enumerate((1, 2)):
@@ -105,9 +108,9 @@ def test_matvec_plane_beyond_shared_memory(prec, tol):
 
 @pytest.mark.parametrize("prec,tol", [("fp64", FP64_TOL), ("fp32", FP32_TOL)])
 def test_matvec_tuned_grid_matches_reference_grid(prec, tol):
-    # box 35 x 40 x 45 with holes: reference grid 70 x 80 x 90 (runtime
-    # plans), tuned grid 80 x 96 x 96 (compile-time plans, fused y/z); the
-    # matvec restricted to the dipoles is the same linear convolution
+    # box 35 x 40 x 45 with holes: reference grid 70 x 80 x 90, tuned grid
+    # 80 x 96 x 96; the matvec restricted to the dipoles is the same linear
+    # convolution
     import dda_b200
     from oracle import oracle as O
     pos = np.array([(x, y, z) for z in range(45) for y in range(40) for x in range(35) if (x * 7 + y * 3 + z) % 11],
@@ -132,19 +135,25 @@ def test_matvec_tuned_grid_matches_reference_grid(prec, tol):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
-@pytest.mark.parametrize("shape", ["box", "sphere"])
-def test_autotuned_layout_gives_identical_results(prec, shape):
-    # the autotuner changes only the batching of the y/z passes: the
-    # product is bit-for-bit the same as with the default layout
+@pytest.mark.parametrize("box,flags,path", [((250, 24, 24), 0, "fused"),                  # grid 500 x 48 x 48
+                                            ((112, 50, 50), api.FLAG_YZ_PAIR, "fused"),   # two CTAs per plane
+                                            ((72, 80, 80), api.FLAG_SLOT_YZ, "cluster")])
+def test_autotuned_layout_gives_identical_results(prec, box, flags, path):
+    # the autotuner changes only the batching of the plane kernels: the
+    # product is bit-for-bit the same as with the default layout (grids of
+    # this test alone: a choice is kept for the process)
     import dda_b200
-    if shape == "box":  # grid 200 x 100 x 100, fused plane kernel
-        g = dda_b200.Geometry.box_shape("5um", "2.5um", "2.5um", "0.05um")
-    else:  # grid 160^3, cluster kernel
-        g = dda_b200.Geometry.sphere("2um", "0.05um")
+    z, y, x = np.meshgrid(*[np.arange(n) for n in box[::-1]], indexing="ij")
+    keep = (x * 7 + y * 3 + z) % 5 < 3
+    keep[0, 0, 0] = keep[-1, -1, -1] = True  # the box's corners
+    pos = np.stack([x[keep], y[keep], z[keep]], axis=1).astype(np.uint32)
+    g = dda_b200.Geometry.from_arrays(pos, np.zeros(len(pos), np.uint8), "0.05um")
     p = dda_b200.DDAParams(g, [1.5 + 0.1j], "1.2um")
-    mvs = [dda_b200.CudaMatVec(p, prec, flags=f) for f in (0, 8)]
+    mvs = [dda_b200.CudaMatVec(p, prec, flags=flags | f) for f in (0, api.FLAG_NO_AUTOTUNE)]
     for mv in mvs:
+        assert mv.layout["yz_path"] == path
         mv.set_couple_constants(dda_b200.CoupleConstants(p, (0, 0, 1), 1, "ldr"))
+    assert mvs[0].launches > mvs[1].launches  # the tuner timed its candidates
     rng = np.random.default_rng(9)
     x = rng.uniform(-1, 1, p.vec_size) + 1j * rng.uniform(-1, 1, p.vec_size)
     for c in range(3):
@@ -159,8 +168,8 @@ def test_autotuned_layout_gives_identical_results(prec, shape):
 def test_grouped_plane_kernel_is_identical(prec, case, groups, pair):
     # the fused plane kernel run as two groups of half the CTA (named
     # barriers, columns and row batches split between the groups) does the
-    # same arithmetic per butterfly: bit-identical to one group, and equal to
-    # the oracle
+    # same arithmetic per butterfly: bit-identical to the grid's own path (one
+    # group at 48 x 48, the three passes beyond), and equal to the oracle
     import dda_b200
     from tests.pairs import Pair
     if case == "cfg1":  # grid 80^3, Plan<10,8>, not half padded
@@ -189,8 +198,11 @@ def test_grouped_plane_kernel_is_identical(prec, case, groups, pair):
             pr = Pair(kind, args, mats, lam, prec, max_rhs=2, flags=flags)
             p, mv, op = pr.p, pr.mv, pr.op
         lay = mv.layout
-        assert lay["yz_path"] == "fused" and lay["groups"] == (groups if flags & gflag else 1)
-        assert lay["ctas_per_plane"] == (2 if pair and flags & gflag else 1)
+        if flags & gflag or case == "half":
+            assert lay["yz_path"] == "fused" and lay["groups"] == (groups if flags & gflag else 1)
+            assert lay["ctas_per_plane"] == (2 if pair and flags & gflag else 1)
+        else:
+            assert lay["yz_path"] == "passes"
         for r, pol in enumerate((1, 2)):
             mv.set_couple_constants(dda_b200.CoupleConstants(p, (0.6, 0.0, 0.8), pol, "ldr"), rhs=r)
         rng = np.random.default_rng(4)
@@ -283,9 +295,9 @@ def test_matvec_batched_rhs(prec, tol):
 
 @pytest.mark.parametrize("prec,tol", [("fp64", FP64_TOL), ("fp32", FP32_TOL)])
 def test_matvec_cfg2_box(prec, tol):
-    # README workload 2: box 10x5x5 um, d = 0.1 um, grid 200x100x100.  The FP64
-    # kx plane (240 KB) exceeds shared memory, so this exercises the split path.
+    # README workload 2: box 10x5x5 um, d = 0.1 um, grid 200x100x100
     pr = Pair("box", ("10um", "5um", "5um", "0.1um"), [1.5 + 0.1j], "6um", prec)
+    assert pr.mv.layout["yz_path"] == "passes"
     pr.set_cc((0, 1, 0), 1, "ldr")
     x = pr.rand_vec(3)
     assert rel(pr.mv.apply(x), pr.op.matvec(x)) < tol

@@ -38,6 +38,7 @@ def test_passes_match_oracle(box, prec, tol):
     mat = (rng.random(len(pos)) < 0.4).astype(np.uint8)
     pr = Pair("arrays", (pos, mat, "0.1um"), [1.5 + 0.1j, 1.3 + 0.02j], "1.1um", prec, max_rhs=3)
     assert pr.p.grid == BOXES[box] and pr.mv.passes == (max(pr.p.grid[1:]) > 42)
+    assert pr.mv.layout["yz_path"] == ("passes" if pr.mv.passes else "fused")
     xs = [pr.rand_vec(40 + r) for r in range(3)]
     want = []
     for r, pol in enumerate((1, 2, 1)):
