@@ -37,6 +37,7 @@ FLAG_NO_AUTOTUNE = 8
 FLAG_YZ_GROUPS2 = 32
 FLAG_YZ_GROUPS4 = 64
 FLAG_YZ_PAIR = 128
+FLAG_SMALL_WORK = 256
 
 
 class Stats(ctypes.Structure):

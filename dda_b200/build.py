@@ -20,7 +20,7 @@ MV_PARTS = [(part, dbl, sub) for dbl in (0, 1) for part in (7, 6, 0, 5, 2, 4, 3,
 HEADERS = ["fft_engine.cuh", "fft_plan.cuh", "reduce.cuh", "krylov_ops.cuh", "krylov_kernels.cuh",
            "matvec_kernels.cuh", "matvec_planned.cuh", "matvec_dispatch.cuh", "dmatrix_kernels.cuh",
            "farfield_kernels.cuh", "matvec_slot.cuh", "kernel_shapes.cuh", "matvec_pair.cuh",
-           "matvec_pass.cuh"]
+           "matvec_pass.cuh", "host_rules.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

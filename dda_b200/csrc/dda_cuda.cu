@@ -32,6 +32,7 @@
 #include "dmatrix_kernels.cuh"
 #include "farfield_kernels.cuh"
 #include "fft_engine.cuh"
+#include "host_rules.h"
 #include "kernel_shapes.cuh"
 #include "krylov_kernels.cuh"
 #include "krylov_ops.cuh"
@@ -538,17 +539,51 @@ inline bool pass_grid(long long Gx, long long Gy, long long Gz, uint32_t flags) 
   return !(small_length((int)Gy) && small_length((int)Gz)) && !(Gy == 48 && Gz == 48);
 }
 
-// Work buffer of the y/z passes: all planes of all right-hand sides, or as
-// much of them as kPassCap holds, and at least the two planes of a frequency
-// for one pair.  y/z passes of the 128-rhs spheroid (4.8 GB in all) with
-// buffers of 64 MB, 256 MB, 1 GB and all: 6.53, 5.72, 5.39, 5.32 ms -- each
-// chunk is three launches with a tail, and staying in L2 does not make up for
-// them; 512^3 (two right-hand sides, 3.2 GB) 6.73, 6.15, 5.93, 5.84 ms.
+// Work buffer of the y/z passes in elements of s bytes: all planes of all
+// right-hand sides, or as much of them as kPassCap holds, and at least the two
+// planes of a frequency, of a pair where pairs run (FP32, max_rhs > 1).  y/z
+// passes of the 128-rhs spheroid (4.8 GB in all) with buffers of 64 MB, 256 MB,
+// 1 GB and all: 6.53, 5.72, 5.39, 5.32 ms -- each chunk is three launches with a
+// tail, and staying in L2 does not make up for them.
+// With DDA_FLAG_SMALL_WORK the buffers of a context's `engines` together take
+// at most 12 bytes per grid point, less than the FP64 grid or the host's D
+// matrix that dda_create frees before it allocates them (both at least that),
+// so that the context's peak is what it would be without them.
 constexpr size_t kPassCap = (size_t)1 << 30;
-inline size_t pass_buffer_bytes(long long Gx, long long Gz, long long by, int max_rhs, size_t s) {
-  const size_t plane = (size_t)(Gz * 3 * by) * s;
-  const size_t all = (size_t)(max_rhs + 1) / 2 * 2 * (2 * (Gx / 2 + 1)) * plane;
-  return std::max(4 * plane, std::min(all, kPassCap));
+inline size_t pass_plane_bytes(long long Gz, long long by, size_t s) { return (size_t)(Gz * 3 * by) * s; }
+inline size_t pass_buffer_least(long long Gz, long long by, int max_rhs, size_t s) {
+  return (s == 8 && max_rhs > 1 ? 4 : 2) * pass_plane_bytes(Gz, by, s);
+}
+inline size_t pass_buffer_bytes(long long Gx, long long Gy, long long Gz, long long by, int max_rhs, size_t s,
+                                uint32_t flags, int engines) {
+  const size_t entries = s == 8 && max_rhs > 1 ? (size_t)(max_rhs + 1) / 2 * 2 : max_rhs;
+  const size_t all = entries * (2 * (Gx / 2 + 1)) * pass_plane_bytes(Gz, by, s);
+  const size_t cap = flags & DDA_FLAG_SMALL_WORK ? (size_t)(12 * Gx * Gy * Gz / engines) : kPassCap;
+  return std::max(pass_buffer_least(Gz, by, max_rhs, s), std::min(all, cap));
+}
+
+// The work buffer of one precision's passes, after everything else the
+// context keeps: where the device is nearly full, half of it, and so on down
+// to the least.
+template <typename T> void alloc_pass_buffer(dda_ctx* c) {
+  Engine<T>& e = eng<T>(c);
+  if (!e.on || !e.pass) return;
+  const MvGeom& g = c->g;
+  const size_t s = sizeof(typename C2<T>::t);
+  const int engines = c->e32.on && c->e64.on ? 2 : 1;
+  e.pbuf_bytes = shrink_to_fit(pass_buffer_bytes(g.Gx, g.Gy, g.Gz, g.by, c->max_rhs, s, c->flags, engines),
+                               pass_buffer_least(g.Gz, g.by, c->max_rhs, s), [&](size_t bytes) {
+    const cudaError_t rc = cudaMallocAsync(&e.pbuf, bytes, c->stream);
+    if (rc == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      e.pbuf = nullptr;
+      return false;
+    }
+    CK(rc);
+    return true;
+  });
+  if (!e.pbuf_bytes) throw DdaError(DDA_ERR_OOM, "no device memory for the work buffer of the y/z passes");
+  g_dalloc_bytes += e.pbuf_bytes;
 }
 
 // The plane kernel of one precision, its tile shapes and buffers: the y/z
@@ -674,8 +709,6 @@ template <typename T> void setup_engine(dda_ctx* c) {
     };
     attrs(e.k.pass1);
     if (c->max_rhs > 1) attrs(e.k.pass2);
-    e.pbuf_bytes = pass_buffer_bytes(g.Gx, g.Gz, g.by, c->max_rhs, s);
-    e.pbuf = dalloc<T>(e.pbuf_bytes);
   }
   const int hx = g.Gx / 2 + 1, hy = g.Gy / 2 + 1, hz = g.Gz / 2 + 1;
   e.dc = (T2*)dalloc<T>((size_t)hx * hy * hz * 6 * s);
@@ -687,11 +720,10 @@ template <typename T> void setup_engine(dda_ctx* c) {
   // convolution in FP32: the FP32 engine needs one input buffer and io
   const bool conv_engine = c->precision == DDA_PREC_MIXED && sizeof(T) == 4;
   const int nvec = conv_engine ? 1 : 10;
-  const size_t vpitch = (vbytes + 255) / 256 * 256;
-  e.vec_bytes = nvec * vpitch;
+  e.vec_bytes = nvec * vbytes;  // vbytes: a multiple of 384 (nvs: of 16)
   e.vec[0] = (T2*)dalloc<T>(e.vec_bytes);
   CK(cudaMemsetAsync(e.vec[0], 0, e.vec_bytes, c->stream));
-  for (int i = 1; i < nvec; i++) e.vec[i] = (T2*)((char*)e.vec[0] + i * vpitch);
+  for (int i = 1; i < nvec; i++) e.vec[i] = (T2*)((char*)e.vec[0] + i * vbytes);
   e.io = (T2*)dalloc<T>(vbytes);
   if (c->precision == DDA_PREC_MIXED && sizeof(T) == 8) {
     e.xo = (T2*)dalloc<T>(vbytes);
@@ -1782,6 +1814,8 @@ int dda_create(const dda_problem* p, int precision, dda_ctx** out) {
     c->cc_set.assign(c->max_rhs, 0);
     if (p->dmatrix) upload_dmatrix(c.get(), p->dmatrix);
     else build_dmatrix(c.get());
+    alloc_pass_buffer<double>(c.get());
+    alloc_pass_buffer<float>(c.get());
     if (!(c->flags & DDA_FLAG_NO_AUTOTUNE)) {
       if (c->e32.on) autotune<float>(c.get());
       // MIXED runs its FP64 engine for a few outer residuals and checks and,
@@ -2273,14 +2307,15 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
   const long long nmat = std::max<uint32_t>(1, p->nmat);
   const bool planned = planned_grid(Gx, Gy, Gz, p->flags);
   long long bytes = 4 * (nl + 1) + 9 * nv;                    // line offsets, dipoles, permutation, materials
-  bytes += 6 * (Gx + Gy + Gz) * (8 + 16 + 4 + 4);              // plans
-  bytes += 4 * (Gx + Gy + Gz) * (8 + 16);                      // their stage twiddles
+  // two plans per axis, one of them with stage twiddles (at most 1.5 tables)
+  bytes += 6 * (Gx + Gy + Gz) * (8 + 16 + 4 + 4);
+  long long work = 0;  // work buffers of the y/z passes
   auto engine = [&](long long s) {
     long long e = (Gx / 2 + 1) * (Gy / 2 + 1) * (Gz / 2 + 1) * 6 * s;  // D-hat octant
     // vectors: 10 Krylov + io; MIXED keeps two more in FP64 (x, b) and only
     // the matvec input and io in FP32
     const long long nvec = precision != DDA_PREC_MIXED ? 11 : s == 16 ? 13 : 2;
-    e += R * nmat * 3 * s + R * Gx * 3 * nl * s + nvec * (R * 3 * nvs * s + 255);
+    e += R * nmat * 3 * s + R * Gx * 3 * nl * s + nvec * R * 3 * nvs * s;
     const long long q = 3 * by + ((3 * by) % 2 == 0 ? 1 : 0);
     const long long smem_yz = (Gz + Gy + Gz * q + 3 * (Gy + 1)) * s;
     bool fused_len = false;
@@ -2289,7 +2324,8 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
 #undef C
     const bool has_yz = !planned || (Gy == Gz && fused_len) || (small_length((int)Gy) && small_length((int)Gz));
     if (pass_grid(Gx, Gy, Gz, p->flags))
-      e += (long long)pass_buffer_bytes(Gx, Gz, by, (int)R, (size_t)s);
+      work += (long long)pass_buffer_bytes(Gx, Gy, Gz, by, (int)R, (size_t)s, p->flags,
+                                           precision == DDA_PREC_MIXED ? 2 : 1);
     else if (!(has_yz && smem_yz <= (long long)kSmemMax) || (p->flags & (DDA_FLAG_SPLIT_YZ | DDA_FLAG_SLOT_YZ)))
       e += R * Gx * 3 * Gz * by * s;
     return e;
@@ -2302,9 +2338,11 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
   const long long tiles = (nl + tl - 1) / tl;
   bytes += R * std::max(3 * tiles, (long long)kVecPartsMax) * (long long)sizeof(RedSums) + R * 4;
   bytes += 2 * R * (long long)sizeof(KrylovState) + R * 100000LL * 8;
-  if (resident) *resident = bytes;
+  if (resident) *resident = bytes + work;
   const long long tmp = p->dmatrix ? (Gx / 2 + 1) * (Gy / 2 + 1) * (Gz / 2 + 1) * 6 * 16 : Gx * Gy * Gz * 16;
-  if (peak) *peak = bytes + tmp;
+  // the work buffers are allocated when `tmp` has been freed; small ones fit in
+  // its place
+  if (peak) *peak = bytes + (p->flags & DDA_FLAG_SMALL_WORK ? std::max(tmp, work) : tmp + work);
   return DDA_OK;
 }
 

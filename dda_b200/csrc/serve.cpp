@@ -1,7 +1,8 @@
 // serve.cpp -- the request loop of include/dda_serve.h.
 //
 // Worker threads (one per slot) take queued requests in arrival order; a
-// request is admitted when its footprint fits the unused budget.  A later,
+// request is admitted when its footprint fits the unused budget, with the small
+// work buffer of the y/z passes where it does not with the full one.  A later,
 // smaller request may go ahead of the head of the queue while the head does
 // not fit, at most kMaxBypass times, after which the head is waited for.
 // Each admitted request runs on its own context and stream: geometry and
@@ -43,7 +44,8 @@ struct Job {
   std::vector<double> refr;
   std::string grid_unit, wavelength;
   dda_problem prob{};
-  int64_t peak = 0;
+  int64_t peak = 0;        // footprint, and with the small work buffer
+  int64_t small_peak = 0;  // (DDA_FLAG_SMALL_WORK)
   double t_submit = 0;
   int bypassed = 0;
 };
@@ -198,16 +200,20 @@ void dda_server::worker() {
           continue;
         }
         auto it = queue.end();
-        if (used + queue.front()->peak <= budget) {
+        if (used + queue.front()->small_peak <= budget) {
           it = queue.begin();
         } else if (queue.front()->bypassed < kMaxBypass) {
           it = std::find_if(queue.begin() + 1, queue.end(),
-                            [&](const std::unique_ptr<Job>& j) { return used + j->peak <= budget; });
+                            [&](const std::unique_ptr<Job>& j) { return used + j->small_peak <= budget; });
           if (it != queue.end()) queue.front()->bypassed++;
         }
         if (it != queue.end()) {
           job = std::move(*it);
           queue.erase(it);
+          if (used + job->peak > budget) {  // rather than waiting for the room
+            job->peak = job->small_peak;
+            job->prob.flags |= DDA_FLAG_SMALL_WORK;
+          }
           break;
         }
         cv_work.wait(lk);  // a finishing request frees budget
@@ -319,12 +325,15 @@ int dda_serve_submit(dda_server* s, const dda_serve_request* q, int64_t* id) {
     return DDA_ERR_ARG;
   }
   int64_t resident = 0;
-  if (dda_footprint(&P, q->precision, &resident, &j->peak) != DDA_OK) {
+  dda_problem small = P;
+  small.flags |= DDA_FLAG_SMALL_WORK;
+  if (dda_footprint(&P, q->precision, &resident, &j->peak) != DDA_OK ||
+      dda_footprint(&small, q->precision, &resident, &j->small_peak) != DDA_OK) {
     g_serve_err = "bad precision";
     return DDA_ERR_ARG;
   }
-  if (j->peak > s->budget) {
-    g_serve_err = "request footprint " + std::to_string(j->peak) + " bytes exceeds the budget of " +
+  if (j->small_peak > s->budget) {
+    g_serve_err = "request footprint " + std::to_string(j->small_peak) + " bytes exceeds the budget of " +
                   std::to_string(s->budget);
     return DDA_ERR_OOM;
   }

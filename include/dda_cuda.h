@@ -104,6 +104,12 @@ typedef struct dda_problem {
  * between this and one CTA per plane; the results are the same); used by
  * tests. */
 #define DDA_FLAG_YZ_PAIR 128u
+/* dda_problem.flags: keep the work buffer of the y/z passes (by default up to
+ * 1 GiB per precision, which is fastest) within the memory that dda_create
+ * needs for a time anyway, so that it adds nothing to the peak (the results are
+ * the same; the request loop sets it where the default does not fit the
+ * budget). */
+#define DDA_FLAG_SMALL_WORK 256u
 
 typedef struct dda_stats {
   int64_t iterations;   /* Krylov iterations (summed over inner solves for MIXED) */
@@ -219,7 +225,9 @@ int dda_choose_grid(const uint32_t* box, int policy, uint32_t* grid);
 
 /* Upper bound of the device memory dda_create(prob, precision) takes:
  * `resident` = what the context keeps, `peak` = resident plus the temporary
- * FP64 grid of the D-matrix generation.  Used to admit requests by HBM
+ * FP64 grid of the D-matrix generation (with DDA_FLAG_SMALL_WORK the work
+ * buffer of the y/z passes takes that grid's place).  Where the device has
+ * less room than `peak`, dda_create makes do with a smaller work buffer.  Used to admit requests by HBM
  * footprint; no counterpart in the reference. */
 int dda_footprint(const dda_problem* prob, int precision, int64_t* resident, int64_t* peak);
 

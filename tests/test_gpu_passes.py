@@ -52,3 +52,33 @@ def test_passes_match_oracle(box, prec, tol):
     assert np.array_equal(pr.mv.apply(xs[0]), three[0])
     assert np.array_equal(pr.mv.apply(np.concatenate(xs[:2])).reshape(2, n), three[:2])
     pr.mv.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32", "mixed"])
+@pytest.mark.parametrize("box,nrhs", [((4, 25, 24), 6),    # room for two entries of one frequency
+                                      ((4, 25, 24), 1),    # ... for several frequencies of one
+                                      ((30, 40, 35), 5)])  # ... for some frequencies of all
+def test_small_work_buffer_gives_identical_results(box, nrhs, prec):
+    # chunks of frequencies and of right-hand sides change no bit
+    import dda_b200
+    from dda_b200 import api
+    z, y, x = np.meshgrid(*[np.arange(n) for n in box[::-1]], indexing="ij")
+    pos = np.stack([v.ravel() for v in (x, y, z)], axis=1).astype(np.uint32)
+    g = dda_b200.Geometry.from_arrays(pos, np.zeros(len(pos), np.uint8), "0.1um")
+    p = dda_b200.DDAParams(g, [1.4 + 0.05j], "2um")
+    rng = np.random.default_rng(nrhs)
+    v = rng.uniform(-1, 1, (nrhs, 3, p.nvs)) + 1j * rng.uniform(-1, 1, (nrhs, 3, p.nvs))
+    v[:, :, p.nv:] = 0
+    out, launches, held = [], [], []
+    for flags in (0, api.FLAG_SMALL_WORK):
+        mv = dda_b200.CudaMatVec(p, prec, max_rhs=nrhs, flags=flags)
+        assert mv.passes
+        for r in range(nrhs):
+            mv.set_couple_constants(dda_b200.CoupleConstants(p, (0, 0.6, 0.8), 1 + r % 2, "ldr"), rhs=r)
+        n = mv.launches
+        out.append(mv.apply(v.ravel()))
+        launches.append(mv.launches - n)
+        held.append(mv.layout["device_bytes"])
+        mv.close()
+    assert np.array_equal(out[0], out[1])
+    assert launches[1] > launches[0] and held[1] < held[0]

@@ -101,3 +101,24 @@ def test_request_beyond_budget_is_rejected():
         _submit(srv, r, 0)
     assert "exceeds the budget" in str(e.value)
     srv.close()
+
+
+def test_request_that_fits_with_the_small_work_buffer_is_accepted():
+    # a budget for the context without its full work buffer: the request is
+    # not refused, and its result has the bits of a context with the buffer
+    pos = targets.spheroid(30, 20, 20)
+    req = dict(positions=pos, materials=None, refr=[1.3 + 0.02j], grid_unit="0.1um", wavelength="2um",
+               prop=(0.0, 0.6, 0.8))
+    done = []
+    for budget in (1 << 30, None):
+        if budget is None:  # what the small buffer needs: less than the first request took
+            budget = done[0]["footprint"] - 1
+        srv = Server(budget_bytes=budget, max_active=1)
+        _submit(srv, req, 0, keep_pol=True)
+        (d,) = srv.drain()
+        srv.close()
+        assert d["status"] == 0, d["error"]
+        assert d["device_bytes"] <= d["footprint"] <= budget
+        done.append(d)
+    assert done[1]["footprint"] < done[0]["footprint"]
+    assert np.array_equal(done[0]["pol"], done[1]["pol"])

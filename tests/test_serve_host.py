@@ -7,8 +7,9 @@ import numpy as np
 from dda_b200 import api, targets
 
 
-def _footprint(grid, box, nv, max_rhs, precision):
+def _footprint(grid, box, nv, max_rhs, precision, flags=0):
     p = api.Problem()
+    p.flags = flags
     p.nv = nv
     p.box = (ctypes.c_uint32 * 3)(*box)
     p.grid = (ctypes.c_uint32 * 3)(*grid)
@@ -30,6 +31,25 @@ def test_footprint_grows_with_rhs_and_precision():
     assert p1 - r1 == 200 * 100 * 100 * 16  # FP64 grid of the D-matrix generation
     # the plane-major x spectrum alone: Gx * 3 * by * bz complex FP32 per rhs
     assert r1 > 200 * 3 * 50 * 50 * 8
+
+
+def test_small_work_buffer_adds_nothing_to_the_peak():
+    # (grid, box, dipoles, right-hand sides) -> peak of a context without the
+    # y/z passes' work buffer: FP32, FP64, mixed
+    plane_kernels = {
+        ((16, 100, 100), (8, 50, 50), 20000, 2): (18110684, 39394364, 48198044),
+        ((8, 50, 48), (4, 25, 24), 2000, 2): (3505932, 4948380, 5910828),
+        ((80, 80, 80), (40, 40, 40), 33510, 2): (37412418, 64563234, 83669250),
+        ((192, 128, 128), (96, 64, 64), 205000, 2): (219659188, 536318740, 652781428),
+        ((192, 128, 128), (96, 64, 64), 205000, 128): (9525296956, 28552197484, 34766498716),
+        ((128, 112, 112), (60, 50, 56), 90000, 1): (69935168, 146840072, 178538576),
+        ((200, 100, 100), (100, 50, 50), 250000, 2): (204662028, 469271724, 577881420),
+    }
+    for c, peaks in plane_kernels.items():
+        for prec, peak in zip(("fp32", "fp64", "mixed"), peaks):
+            small, full = (_footprint(*c, prec, flags=f) for f in (api.FLAG_SMALL_WORK, 0))
+            assert small[1] <= peak, (c, prec)
+            assert small[0] <= small[1] and small[0] <= full[0] and small[1] < full[1], (c, prec)
 
 
 def test_spheroid_matches_cell_centre_count():
