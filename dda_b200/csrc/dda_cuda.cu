@@ -2436,32 +2436,40 @@ void far_field_few(dda_ctx* c, int nrhs, const double* ddirs, long long ndir, do
   c->launches++;
 }
 
-// part: room for part_bytes of partial sums.
+// Splits of the lines: about eight waves of CTAs, at least two lines per warp,
+// or eight where the directions alone fill half the SMs, as each split
+// computes its x phases again (21 x 12 x 14, 2 978 directions: ten splits
+// 220 us, two 177).
+template <int NR, int DL> int ff_splits(dda_ctx* c, int nrhs, long long ndir) {
+  int nsm = 148;
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+  const int nd = 32 * DL;
+  const long long ctas = (ndir + nd - 1) / nd * ((nrhs + NR - 1) / NR);
+  const int lines = 2 * ctas >= nsm ? 8 : 2;
+  return (int)std::max<long long>(
+      1, std::min<long long>({(16LL / DL * nsm + ctas - 1) / ctas, 64, c->g.nlines / (lines * (kNtFf / 32))}));
+}
+
+// part: room for part_bytes of partial sums.  As many of the `splits` as there
+// is room for with all directions in one launch; blocks of directions, one
+// split, where there is none for all of them.  (More splits and blocks of
+// fewer directions would keep the CTAs of a launch and add launches.)
 template <typename T, int NR, int DL>
-void far_field_many(dda_ctx* c, int nrhs, const double* ddirs, long long ndir, double2* dout, double2* part,
-                    size_t part_bytes) {
+void far_field_many(dda_ctx* c, int nrhs, const double* ddirs, long long ndir, double2* dout, int splits,
+                    double2* part, size_t part_bytes) {
   const FfGeom g = far_field_geom(c);
   const size_t smem = ff_part_smem<NR, DL>(g.bx), row = (size_t)nrhs * 3 * sizeof(double2);
   CK(allow_smem((const void*)k_ff_part<T, NR, DL>));
-  int nsm = 148;
-  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
   const int zr = (nrhs + NR - 1) / NR, nd = 32 * DL;
-  // directions per launch and splits of the lines: about eight waves of CTAs,
-  // within the room; at least two lines per warp, or eight where the
-  // directions alone fill half the SMs, as each split computes its x phases
-  // again (21 x 12 x 14, 2 978 directions: ten splits 220 us, two 177)
   const long long fit = std::max<long long>(1, (long long)(part_bytes / row));
-  const long long ctas = (std::min(ndir, fit) + nd - 1) / nd * zr;
-  long long splits = (16LL / DL * nsm + ctas - 1) / ctas;
-  const int lines = 2 * ctas >= nsm ? 8 : 2;
-  splits = std::max<long long>(1, std::min<long long>({splits, 64, g.nlines / (lines * (kNtFf / 32)), fit / nd}));
-  const long long block = std::min<long long>(ndir, fit / splits);
+  splits = (int)std::max<long long>(1, std::min<long long>(splits, fit / ndir));
+  const long long block = std::min(ndir, fit);
   for (long long d0 = 0; d0 < ndir; d0 += block) {
     const int n = (int)std::min(block, ndir - d0);
-    k_ff_part<T, NR, DL><<<dim3((n + nd - 1) / nd, (unsigned)splits, zr), kNtFf, smem, c->stream>>>(
+    k_ff_part<T, NR, DL><<<dim3((n + nd - 1) / nd, splits, zr), kNtFf, smem, c->stream>>>(
         eng<T>(c).io, c->line_off, c->dip, c->perm, ddirs + 3 * d0, n, nrhs, g, part);
     k_ff_combine<<<(unsigned)(((long long)n * nrhs + 127) / 128), 128, 0, c->stream>>>(
-        part, (int)splits, ddirs + 3 * d0, n, nrhs, g, dout + (size_t)d0 * nrhs * 3);
+        part, splits, ddirs + 3 * d0, n, nrhs, g, dout + (size_t)d0 * nrhs * 3);
     c->launches += 2;
   }
   CK(cudaGetLastError());
@@ -2481,12 +2489,15 @@ void far_field_t(dda_ctx* c, int nrhs, const double* pol, long long ndir, const 
   const size_t obytes = ((size_t)ndir * nrhs * 3 * sizeof(double2) + 255) / 256 * 256;
   const bool many = ndir >= (c->g.nlines > 256 ? kFfFew : 2 * kFfFew) && ff_part_smem<2, 1>(c->g.bx) <= kSmemMax;
   const bool two = nrhs == 1 && ndir >= kFfTwo && ff_part_smem<1, 2>(c->g.bx) <= kSmemMax;
+  const int splits = !many ? 0
+                     : two ? ff_splits<1, 2>(c, nrhs, ndir)
+                     : nrhs == 1 ? ff_splits<1, 1>(c, nrhs, ndir) : ff_splits<2, 1>(c, nrhs, ndir);
   const size_t least = many ? std::min(obytes, kFfPartBytes) : 0;  // one split of the lines
   char* buf = (char*)e.vec[0];
   size_t room = e.vec_bytes;
   void* temp = nullptr;
   if (dbytes + obytes + least > room) {
-    room = dbytes + obytes + least;
+    room = dbytes + obytes + std::min(splits * obytes, kFfPartBytes);
     CK(cudaMallocAsync(&temp, room, c->stream));
     buf = (char*)temp;
   }
@@ -2496,9 +2507,9 @@ void far_field_t(dda_ctx* c, int nrhs, const double* pol, long long ndir, const 
   const size_t part_bytes = room - dbytes - obytes;
   CK(cudaMemcpyAsync(ddirs, dirs, ndir * 3 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   if (!many) far_field_few<T>(c, nrhs, ddirs, ndir, dout);
-  else if (two) far_field_many<T, 1, 2>(c, nrhs, ddirs, ndir, dout, part, part_bytes);
-  else if (nrhs == 1) far_field_many<T, 1, 1>(c, nrhs, ddirs, ndir, dout, part, part_bytes);
-  else far_field_many<T, 2, 1>(c, nrhs, ddirs, ndir, dout, part, part_bytes);
+  else if (two) far_field_many<T, 1, 2>(c, nrhs, ddirs, ndir, dout, splits, part, part_bytes);
+  else if (nrhs == 1) far_field_many<T, 1, 1>(c, nrhs, ddirs, ndir, dout, splits, part, part_bytes);
+  else far_field_many<T, 2, 1>(c, nrhs, ddirs, ndir, dout, splits, part, part_bytes);
   CK(cudaMemcpyAsync(out, dout, (size_t)ndir * nrhs * 3 * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
   if (temp) CK(cudaFreeAsync(temp, c->stream));
   CK(cudaStreamSynchronize(c->stream));

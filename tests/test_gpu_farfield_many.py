@@ -1,8 +1,7 @@
-"""The far field of many directions (k_ff_part) against the oracle's sum and
-against the few-direction kernel, on both sides of the rule's thresholds and at
-the edges of its 32- and 64-direction blocks, with one to three right-hand
-sides (pairs and a remainder), permuted dipoles and a request beyond the
-context's workspace."""
+"""The far field of many directions (k_ff_part) against the sum over the dipoles
+in NumPy, on both sides of the rule's thresholds and at the edges of its 32- and
+64-direction blocks, with one to three right-hand sides (pairs and a remainder),
+permuted dipoles and requests beyond the context's workspace."""
 import numpy as np
 import pytest
 
@@ -48,4 +47,43 @@ def test_far_field_of_many_directions(prec, target, ndir):
         got = mv.far_field(dirs, nrhs=n, pol=pol[:n])
         # sums of 120 to 4 200 terms of phases up to 20 rad in FP64, in another order
         assert np.abs(got - want[:, :n]).max() < 1e-12 * np.abs(want).max()
+    mv.close()
+
+
+def test_splits_of_a_small_target_take_one_launch():
+    # 400 lines, 2 978 directions: 25 splits of the lines want 25 sets of
+    # partial sums, beyond the Krylov vectors' room; all directions still go in
+    # one launch (and one that adds the sums)
+    g = dda_b200.Geometry.sphere("1um", "0.1um")
+    p = dda_b200.DDAParams(g, [1.5 + 0.1j], "0.9um")
+    rng = np.random.default_rng(1)
+    dirs = rng.normal(size=(2978, 3))
+    dirs /= np.linalg.norm(dirs, axis=1, keepdims=True)
+    for nrhs in (1, 2):
+        mv = dda_b200.CudaMatVec(p, "fp64", max_rhs=nrhs)
+        pol = rng.uniform(-1, 1, (nrhs, p.vec_size)) + 1j * rng.uniform(-1, 1, (nrhs, p.vec_size))
+        want = _sum(p, pol, dirs)
+        n = mv.launches
+        got = mv.far_field(dirs, nrhs=nrhs, pol=pol)
+        assert mv.launches - n == 2
+        assert np.abs(got - want).max() < 1e-12 * np.abs(want).max()
+        mv.close()
+
+
+def test_directions_beyond_the_room_go_in_blocks():
+    # one set of partial sums is 67 MB, above the 64 MB of a request that
+    # allocates: two blocks of directions
+    g = dda_b200.Geometry.from_arrays(*scrambled_arrays())
+    p = dda_b200.DDAParams(g, [1.5 + 0.1j, 1.3 + 0.0j], "0.9um")
+    mv = dda_b200.CudaMatVec(p, "fp64", max_rhs=2)
+    rng = np.random.default_rng(2)
+    dirs = rng.normal(size=(700000, 3))
+    dirs /= np.linalg.norm(dirs, axis=1, keepdims=True)
+    pol = rng.uniform(-1, 1, (2, p.vec_size)) + 1j * rng.uniform(-1, 1, (2, p.vec_size))
+    n = mv.launches
+    got = mv.far_field(dirs, nrhs=2, pol=pol)
+    assert mv.launches - n == 4
+    for at in (slice(0, 100), slice(699000, 699100), slice(-100, None)):  # the second block begins at 699 050
+        want = _sum(p, pol, dirs[at])
+        assert np.abs(got[at] - want).max() < 1e-12 * np.abs(want).max()
     mv.close()
