@@ -2397,15 +2397,32 @@ int dda_profile_matvec(dda_ctx* ctx, int nrhs, int reps, double* ms) {
 namespace {
 // The far field of e.io: k_farfield for a few directions, whose lines are
 // then the only parallelism, or where the x phases of 32 directions do not
-// fit shared memory; else k_ff_part, directions on the lanes.
-// Threshold: 40^3 sphere, FP64, both polarisations: 31 directions 177 us with
-// k_farfield, 32 with k_ff_part 128 (5 551: 1 653 -> 745); with at most one
-// line per thread (14 x 14 x 10) k_farfield is as fast up to 56 (50 to 56 us).
+// fit shared memory; else k_ff_part, directions on the lanes (ff_on_lanes).
 // Two directions per lane help where a lane has one right-hand side (40^3,
 // FP32, 5 551 directions: 471 -> 418 us; 1 024: 196 -> 178), not two, which
 // give a read 24 FMAs already (744 and 770).
-constexpr int kFfFew = 32, kFfTwo = 1024;
+constexpr int kFfTwo = 1024;
 constexpr size_t kFfPartBytes = (size_t)64 << 20;  // of a request that allocates
+
+// Whether k_ff_part takes a request.  From 32 directions on where the lines
+// are more than k_farfield's threads (40^3 sphere, FP64, both polarisations:
+// 32 directions 173 us with k_farfield, 122 with k_ff_part; 3 600: 1 146 and
+// 528).  With a line per thread at most, k_farfield takes the same time up to
+// one CTA (four directions, one right-hand side) per SM, which is then shorter
+// (14 x 14 x 10, both polarisations: 64 to 192 directions 41 to 44 and 44 to
+// 50 us, 384 55 and 53, 1 600 99 and 82; 7 x 7 x 10: 192 46 and 52, 1 100 91
+// and 83) unless the lines are long and k_ff_part's warps have some each
+// (100 x 8 x 8, one polarisation: 64 directions 80 and 58; 100 x 16 x 16, both:
+// 128 and 110; but 200 x 6 x 6, both: 112 and 125).
+bool ff_on_lanes(const dda_ctx* c, int nrhs, long long ndir) {
+  if (ff_part_smem<2, 1>(c->g.bx) > kSmemMax) return false;
+  if (c->g.nlines > 256) return ndir >= 32;
+  if (ndir < 64) return false;
+  if (c->g.bx > 64 && (nrhs == 1 || c->g.nlines >= 64)) return true;
+  int nsm = 148;
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+  return ndir * nrhs > 4LL * nsm;
+}
 
 FfGeom far_field_geom(const dda_ctx* c) {
   FfGeom g;
@@ -2487,7 +2504,7 @@ void far_field_t(dda_ctx* c, int nrhs, const double* pol, long long ndir, const 
   // beyond them allocates
   const size_t dbytes = ((size_t)ndir * 3 * sizeof(double) + 255) / 256 * 256;
   const size_t obytes = ((size_t)ndir * nrhs * 3 * sizeof(double2) + 255) / 256 * 256;
-  const bool many = ndir >= (c->g.nlines > 256 ? kFfFew : 2 * kFfFew) && ff_part_smem<2, 1>(c->g.bx) <= kSmemMax;
+  const bool many = ff_on_lanes(c, nrhs, ndir);
   const bool two = nrhs == 1 && ndir >= kFfTwo && ff_part_smem<1, 2>(c->g.bx) <= kSmemMax;
   const int splits = !many ? 0
                      : two ? ff_splits<1, 2>(c, nrhs, ndir)

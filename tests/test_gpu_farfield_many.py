@@ -87,3 +87,31 @@ def test_directions_beyond_the_room_go_in_blocks():
         want = _sum(p, pol, dirs[at])
         assert np.abs(got[at] - want).max() < 1e-12 * np.abs(want).max()
     mv.close()
+
+
+def test_kernel_of_a_request():
+    # k_farfield is one launch, k_ff_part two: the rule's lines for a small
+    # target, a long one and one of more than 256 lines
+    torch = pytest.importorskip("torch")
+    wave = 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    long_box = np.stack([v.ravel() for v in np.meshgrid(np.arange(100), np.arange(8), np.arange(8), indexing="ij")],
+                        axis=1).astype(np.uint32)
+    long_box = long_box[np.lexsort((long_box[:, 0], long_box[:, 1], long_box[:, 2]))]
+    small = dda_b200.Geometry.from_arrays(*scrambled_arrays())
+    cases = [(small, 2, wave // 2), (small, 1, wave),
+             (dda_b200.Geometry.from_arrays(long_box, np.zeros(len(long_box), np.uint8), "0.1um"), 1, 63),
+             (dda_b200.Geometry.sphere("1um", "0.1um"), 2, 31)]
+    rng = np.random.default_rng(3)
+    for g, nrhs, last_few in cases:
+        p = dda_b200.DDAParams(g, [1.5 + 0.1j, 1.3 + 0.0j] if g is small else [1.5 + 0.1j], "0.9um")
+        mv = dda_b200.CudaMatVec(p, "fp64", max_rhs=nrhs)
+        pol = rng.uniform(-1, 1, (nrhs, p.vec_size)) + 1j * rng.uniform(-1, 1, (nrhs, p.vec_size))
+        for ndir, launches in ((last_few, 1), (last_few + 1, 2)):
+            dirs = rng.normal(size=(ndir, 3))
+            dirs /= np.linalg.norm(dirs, axis=1, keepdims=True)
+            n = mv.launches
+            got = mv.far_field(dirs, nrhs=nrhs, pol=pol)
+            assert mv.launches - n == launches, (nrhs, ndir)
+            want = _sum(p, pol, dirs)
+            assert np.abs(got - want).max() < 1e-12 * np.abs(want).max()
+        mv.close()
