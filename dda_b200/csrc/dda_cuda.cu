@@ -1388,38 +1388,6 @@ bool check_gap(dda_ctx* c, int nrhs, double2* X, double2* B, double2* tmp, const
   return all;
 }
 
-// Iterations of the next round: `poll`, or fewer when every running right-hand
-// side is expected to converge within them.  A kernel whose right-hand sides
-// are all done still costs its launch (a BiCGStab iteration of the two-rhs box
-// 43 us of about 240), a look at the flags some 20 us.  The expectation is the
-// mean rate of the residual since the last look; a round is an even number of
-// iterations (RoundGraph), and rounds end on multiples of `poll` wherever they
-// are not cut short, so that what is done every so many iterations is done at
-// the same ones.
-struct RoundLength {
-  std::vector<double> last;
-  long long last_nr = 0;
-  RoundLength(const KrylovState* st, int nrhs) : last(nrhs, 0.0) {
-    for (int r = 0; r < nrhs; r++) last[r] = st[r].inprodR;
-  }
-  int update(const KrylovState* st, long long nr, int poll) {
-    const int full = poll - (int)(nr % poll);
-    double need = 0;
-    for (size_t r = 0; r < last.size(); r++) {
-      const KrylovState& k = st[r];
-      const double now = k.inprodR;
-      if (!k.done) {
-        const double rate = nr > last_nr && last[r] > now ? std::log(last[r] / now) / (double)(nr - last_nr) : 0.0;
-        need = std::max(need, rate > 0 && k.epsB > 0 ? std::log(now / k.epsB) / rate : (double)full);
-      }
-      last[r] = now;
-    }
-    last_nr = nr;
-    if (!(need < full)) return full;
-    return std::max(2, std::min(full, 2 * (int)std::ceil(need / 2)));
-  }
-};
-
 // Runs one solve of `nrhs` right-hand sides already set up in the engine
 // vectors (E = einc or B = b, S = start).  Per-rhs states end in c->st_host;
 // the solution x is left in engine vector 4.
@@ -1474,7 +1442,7 @@ void run_solve(dda_ctx* c, int solver, int nrhs, double eps, long long max_iter,
   // captured order; all other kernel arguments are fixed pointers, and the
   // kernels read their scalars and done flags from the device state.
   const int poll = 8, per_graph = 2;
-  RoundLength next_round(c->st_host, nrhs);
+  RoundLength<KrylovState> next_round(c->st_host, nrhs);
   const bool graphs = !(c->flags & DDA_FLAG_NO_GRAPHS);
   // graph of the current kernel sequence (index into c->round_graphs, which
   // may grow while this solve runs: a precision switch captures a second one)
