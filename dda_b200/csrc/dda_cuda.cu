@@ -520,11 +520,10 @@ inline bool planned_grid(long long Gx, long long Gy, long long Gz, uint32_t flag
 }
 
 // Whether a grid's y/z passes run as the three kernels of matvec_pass.cuh,
-// instead of a plane kernel.  Whole matvec, one / two right-hand sides, FP32
-// unless said, kernels replayed from a graph; against the planned plane
-// kernels of the tuned lengths: 56^3 24.8 -> 21.3 / 25.2 -> 23.8 us, 80^3
-// 34.7 -> 29.1 / 57.2 -> 36.8, 128^3 79.8 -> 54.9 / 148 -> 91, 200^3 472 -> 214
-// / 876 -> 420; FP64 80^3 55.3 -> 39.2 / 97.6 -> 58.0; against the
+// instead of a plane kernel (but for plane_wave).  Whole matvec, one / two
+// right-hand sides, FP32 unless said, kernels replayed from a graph; against
+// the planned plane kernels of the tuned lengths: 80^3 34.7 -> 29.1 / 57.2 ->
+// 36.8 us, 128^3 79.8 -> 54.9 / 148 -> 91, 200^3 472 -> 214 / 876 -> 420; FP64 80^3 55.3 -> 39.2 / 97.6 -> 58.0; against the
 // runtime-planned one, 50^3 52.1 -> 20.3.  Small planes are one small CTA of
 // k_yz_p each, and two launches more cost what the passes gain: replayed,
 // passes and plane kernel 10^3 14.1 and 11.9, 30^3 17.3 and 16.1, 42^3 19.3 and
@@ -537,6 +536,27 @@ inline bool pass_grid(long long Gx, long long Gy, long long Gz, uint32_t flags) 
     return false;
   if (!has_plan((int)Gx) || !has_plan((int)Gy) || !has_plan((int)Gz)) return false;
   return !(small_length((int)Gy) && small_length((int)Gz)) && !(Gy == 48 && Gz == 48);
+}
+
+// Where a grid of the passes still runs its plane kernel for nrhs right-hand
+// sides of s-byte elements: 56 x 56 planes and, in FP32, 64 x 64, that are one
+// wave of k_yz_p's CTAs, one per SM, and fill a good part of it.  y/z of 56 x 56,
+// passes and plane kernel: FP32 56 planes 18.4 and 19.0 us, 112 22.1 and 18.8,
+// 224 25.6 and 31.1; FP64 22.8 and 22.9, 27.6 and 22.9, 39.9 and 40.6.  BiCGStab
+// on 56^3, both polarisations: FP32 861 and 766 us, FP64 924 and 844; on 64^3
+// FP32 917 and 876.
+inline bool plane_wave(long long Gx, long long Gy, long long Gz, int nrhs, size_t s) {
+  constexpr int kSms = 148;
+  if (Gy != Gz || !(Gy == 56 || (Gy == 64 && s == 8))) return false;
+  return Gx * nrhs >= 56 && Gx * nrhs <= kSms;
+}
+// Whether some of 1 to max_rhs right-hand sides run it, and all of them.
+inline bool plane_wave_some(long long Gx, long long Gy, long long Gz, int max_rhs, size_t s) {
+  const int n = (int)std::max(1LL, (55 + Gx) / Gx);  // the fewest of 56 planes
+  return n <= max_rhs && plane_wave(Gx, Gy, Gz, n, s);
+}
+inline bool plane_wave_all(long long Gx, long long Gy, long long Gz, int max_rhs, size_t s) {
+  return plane_wave(Gx, Gy, Gz, 1, s) && plane_wave(Gx, Gy, Gz, max_rhs, s);
 }
 
 // Work buffer of the y/z passes in elements of s bytes: all planes of all
@@ -678,8 +698,9 @@ template <typename T> void setup_engine(dda_ctx* c) {
   const size_t s = sizeof(T2);
   e.on = true;
   e.k = select_kernels<T>(c->planned, g.Gx, g.Gy, g.Gz, g.by, g.bz);
-  e.pass = pass_grid(g.Gx, g.Gy, g.Gz, c->flags);
-  if (!e.pass) setup_plane<T>(c);
+  const bool passes = pass_grid(g.Gx, g.Gy, g.Gz, c->flags);
+  e.pass = passes && !plane_wave_all(g.Gx, g.Gy, g.Gz, c->max_rhs, s);
+  if (!passes || plane_wave_some(g.Gx, g.Gy, g.Gz, c->max_rhs, s)) setup_plane<T>(c);
   pick_x_tile<T>(c, e);
   if (e.smem_x > kSmemMax) throw DdaError(DDA_ERR_UNSUPPORTED, "grid x extent too large");
   // (a kernel that stays within the 48 KB every kernel may use is not looked
@@ -788,6 +809,12 @@ int launch_pass(dda_ctx* c, const PassKernels<T, W>& k, int nrhs, cudaStream_t s
   return launches;
 }
 
+// Whether nrhs right-hand sides run the passes, not the plane kernel.
+template <typename T> bool runs_passes(const dda_ctx* c, int nrhs) {
+  const Engine<T>& e = eng<T>(const_cast<dda_ctx*>(c));
+  return e.pass && !(e.fused && plane_wave(c->g.Gx, c->g.Gy, c->g.Gz, nrhs, sizeof(typename C2<T>::t)));
+}
+
 // The y/z passes: the kernels of matvec_pass.cuh, or the fused plane kernel,
 // the cluster kernel or the split path (column FFTs along z around the row
 // kernel).  Returns the number of launches.
@@ -796,7 +823,7 @@ int launch_yz(dda_ctx* c, int nrhs, cudaStream_t s, KrylovState* st, int skipmv)
   Engine<T>& e = eng<T>(c);
   const MvGeom& g = c->g;
   const FftPlanDev py = c->my.dev<T>(), pz = c->mz.dev<T>();
-  if (e.pass) {
+  if (runs_passes<T>(c, nrhs)) {
     if constexpr (sizeof(T) == 4)
       if (nrhs > 1 && e.k.pass2.zfwd && e.k.pass2.rows)
         return launch_pass<T, 2>(c, e.k.pass2, nrhs, s, st, skipmv);
@@ -2291,7 +2318,7 @@ int dda_footprint(const dda_problem* p, int precision, int64_t* resident, int64_
     DDA_FUSED_LENGTHS(C)
 #undef C
     const bool has_yz = !planned || (Gy == Gz && fused_len) || (small_length((int)Gy) && small_length((int)Gz));
-    if (pass_grid(Gx, Gy, Gz, p->flags))
+    if (pass_grid(Gx, Gy, Gz, p->flags) && !plane_wave_all(Gx, Gy, Gz, (int)R, (size_t)s))
       work += (long long)pass_buffer_bytes(Gx, Gy, Gz, by, (int)R, (size_t)s, p->flags,
                                            precision == DDA_PREC_MIXED ? 2 : 1);
     else if (!(has_yz && smem_yz <= (long long)kSmemMax) || (p->flags & (DDA_FLAG_SPLIT_YZ | DDA_FLAG_SLOT_YZ)))
@@ -2325,8 +2352,8 @@ int dda_matvec_layout(const dda_ctx* ctx, int64_t* out) {
     out[3] = side_by_side;
     out[4] = (int64_t)k.smem_rows;
   };
-  auto fill = [&](const auto& e) {
-    if (e.pass) {
+  auto fill = [&](const auto& e, bool passes) {
+    if (passes) {
       if (ctx->max_rhs > 1 && e.k.pass2.zfwd && e.k.pass2.rows) pass(e.k.pass2, 2);
       else pass(e.k.pass1, 1);
       return;
@@ -2337,8 +2364,8 @@ int dda_matvec_layout(const dda_ctx* ctx, int64_t* out) {
     out[3] = e.slot_path ? e.sg.nrw : e.yz.nrw;
     out[4] = (int64_t)(e.fused ? e.smem_yz : e.slot_path ? e.smem_slot : e.smem_rows);
   };
-  if (ctx->e32.on) fill(ctx->e32);
-  else fill(ctx->e64);
+  if (ctx->e32.on) fill(ctx->e32, runs_passes<float>(ctx, ctx->max_rhs));
+  else fill(ctx->e64, runs_passes<double>(ctx, ctx->max_rhs));
   out[5] = ctx->e32.on ? ctx->e32.tl : ctx->e64.tl;
   out[6] = ctx->planned ? 1 : 0;
   out[7] = (int64_t)ctx->dev_bytes;
@@ -2347,7 +2374,7 @@ int dda_matvec_layout(const dda_ctx* ctx, int64_t* out) {
 
 int dda_matvec_passes(const dda_ctx* ctx) {
   if (!ctx) return 0;
-  return (ctx->e32.on ? ctx->e32.pass : ctx->e64.pass) ? 1 : 0;
+  return (ctx->e32.on ? runs_passes<float>(ctx, ctx->max_rhs) : runs_passes<double>(ctx, ctx->max_rhs)) ? 1 : 0;
 }
 
 int dda_profile_matvec(dda_ctx* ctx, int nrhs, int reps, double* ms) {

@@ -231,8 +231,9 @@ int dda_choose_grid(const uint32_t* box, int policy, uint32_t* grid);
  * footprint; no counterpart in the reference. */
 int dda_footprint(const dda_problem* prob, int precision, int64_t* resident, int64_t* peak);
 
-/* Layout the context chose for its matvec (working precision: FP32 for
- * DDA_PREC_FP32 and DDA_PREC_MIXED, FP64 otherwise), 8 values:
+/* Layout the context chose for its matvec of max_rhs right-hand sides (working
+ * precision: FP32 for DDA_PREC_FP32 and DDA_PREC_MIXED, FP64 otherwise), 8
+ * values:
  * [0] y/z path (0 fused plane kernel, 1 cluster kernel, 2 split path, 3 the
  * passes: three kernels over a work buffer),
  * [1] resident clusters (cluster kernel), CTAs per kx plane (fused kernels:
@@ -247,7 +248,8 @@ int dda_footprint(const dda_problem* prob, int precision, int64_t* resident, int
  * benchmark reports; no counterpart in the reference. */
 int dda_matvec_layout(const dda_ctx* ctx, int64_t* out);
 
-/* 1 when the context's matvecs (working precision) run their y/z passes as
+/* 1 when the context's matvecs of max_rhs right-hand sides (working precision)
+ * run their y/z passes as
  * the three kernels z forward, y rows with the D multiply, z inverse over a
  * work buffer (dda_matvec_layout [0] = 3), 0 when they run a plane kernel.  A
  * diagnostic; no counterpart in the reference. */

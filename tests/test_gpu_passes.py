@@ -82,3 +82,43 @@ def test_small_work_buffer_gives_identical_results(box, nrhs, prec):
         mv.close()
     assert np.array_equal(out[0], out[1])
     assert launches[1] > launches[0] and held[1] < held[0]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32", "mixed"])
+@pytest.mark.parametrize("box", [(28, 28, 28), (9, 28, 28), (64, 28, 28), (32, 32, 32), (75, 32, 32)])
+def test_one_wave_of_planes(box, prec):
+    # 56 x 56 planes (FP32: 64 x 64 too) run the plane kernel for the batches
+    # of which they are one wave, the passes for others: the same bits
+    import dda_b200
+    from dda_b200 import api
+    z, y, x = np.meshgrid(*[np.arange(n) for n in box[::-1]], indexing="ij")
+    pos = np.stack([v.ravel() for v in (x, y, z)], axis=1).astype(np.uint32)
+    g = dda_b200.Geometry.from_arrays(pos, np.zeros(len(pos), np.uint8), "0.1um")
+    p = dda_b200.DDAParams(g, [1.4 + 0.05j], "2um")
+    gx, small = p.grid[0], p.grid[1] == 56 or prec != "fp64"
+    assert p.grid[1:] == (2 * box[1], 2 * box[2])
+    wave = [small and 56 <= gx * n <= 148 for n in range(1, 5)]
+    rng = np.random.default_rng(2)
+    v = rng.uniform(-1, 1, (4, 3, p.nvs)) + 1j * rng.uniform(-1, 1, (4, 3, p.nvs))
+    v[:, :, p.nv:] = 0
+    v = v.reshape(4, -1)
+
+    def products(max_rhs, flags=0):
+        mv = dda_b200.CudaMatVec(p, prec, max_rhs=max_rhs, flags=flags)
+        assert flags or mv.passes == (not wave[max_rhs - 1])
+        for r in range(max_rhs):
+            mv.set_couple_constants(dda_b200.CoupleConstants(p, (0, 0.6, 0.8), 1 + r % 2, "ldr"), rhs=r)
+        out = []
+        for n in range(1, max_rhs + 1):
+            k = mv.launches
+            out.append(mv.apply(v[:n].ravel()))
+            # (an apply in mixed precision is FP64)
+            if not flags and prec != "mixed":
+                assert mv.launches - k == (3 if wave[n - 1] else 5) + (4 if prec == "fp32" else 0), n
+        mv.close()
+        return out
+
+    want = products(4, api.FLAG_YZ_GROUPS2 if p.grid[0] in (56, 64, 128) else 0)  # (tuned lengths)
+    for max_rhs in (1, 2, 4):
+        for a, b in zip(products(max_rhs), want):
+            assert np.array_equal(a, b)
