@@ -582,26 +582,36 @@ inline size_t pass_buffer_bytes(long long Gx, long long Gy, long long Gz, long l
   return std::max(pass_buffer_least(Gz, by, max_rhs, s), std::min(all, cap));
 }
 
+// Allocates on the context's stream; false where the device has no room.
+bool try_alloc(dda_ctx* c, void** p, size_t bytes) {
+  const cudaError_t rc = cudaMallocAsync(p, bytes, c->stream);
+  if (rc == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    *p = nullptr;
+    return false;
+  }
+  CK(rc);
+  return true;
+}
+
+// Bytes that one precision's work buffer should have, 0 for none.
+template <typename T> size_t pass_buffer_wanted(dda_ctx* c) {
+  Engine<T>& e = eng<T>(c);
+  if (!e.on || !e.pass) return 0;
+  const MvGeom& g = c->g;
+  return pass_buffer_bytes(g.Gx, g.Gy, g.Gz, g.by, c->max_rhs, sizeof(typename C2<T>::t), c->flags,
+                           c->e32.on && c->e64.on ? 2 : 1);
+}
+
 // The work buffer of one precision's passes, after everything else the
 // context keeps: where the device is nearly full, half of it, and so on down
 // to the least.
 template <typename T> void alloc_pass_buffer(dda_ctx* c) {
   Engine<T>& e = eng<T>(c);
-  if (!e.on || !e.pass) return;
-  const MvGeom& g = c->g;
-  const size_t s = sizeof(typename C2<T>::t);
-  const int engines = c->e32.on && c->e64.on ? 2 : 1;
-  e.pbuf_bytes = shrink_to_fit(pass_buffer_bytes(g.Gx, g.Gy, g.Gz, g.by, c->max_rhs, s, c->flags, engines),
-                               pass_buffer_least(g.Gz, g.by, c->max_rhs, s), [&](size_t bytes) {
-    const cudaError_t rc = cudaMallocAsync(&e.pbuf, bytes, c->stream);
-    if (rc == cudaErrorMemoryAllocation) {
-      cudaGetLastError();
-      e.pbuf = nullptr;
-      return false;
-    }
-    CK(rc);
-    return true;
-  });
+  const size_t want = pass_buffer_wanted<T>(c);
+  if (!want) return;
+  e.pbuf_bytes = shrink_to_fit(want, pass_buffer_least(c->g.Gz, c->g.by, c->max_rhs, sizeof(typename C2<T>::t)),
+                               [&](size_t bytes) { return try_alloc(c, &e.pbuf, bytes); });
   if (!e.pbuf_bytes) throw DdaError(DDA_ERR_OOM, "no device memory for the work buffer of the y/z passes");
   g_dalloc_bytes += e.pbuf_bytes;
 }
@@ -1045,8 +1055,12 @@ void build_dmatrix(dda_ctx* c) {
   NvtxRange range("dda D matrix");
   const MvGeom& g = c->g;
   const long long N = (long long)g.Gx * g.Gy * g.Gz;
+  // as large as the larger work buffer of the passes where there is room: that
+  // then takes the block over (mapping new memory costs 5 ms a GB)
   double2* full = nullptr;
-  CK(cudaMallocAsync(&full, N * sizeof(double2), c->stream));
+  const size_t bytes = N * sizeof(double2);
+  const size_t later = std::max(pass_buffer_wanted<double>(c), pass_buffer_wanted<float>(c));
+  if (later <= bytes || !try_alloc(c, (void**)&full, later)) CK(cudaMallocAsync(&full, bytes, c->stream));
   const FftPlanDev px = c->px.dev<double>(), py = c->py.dev<double>(), pz = c->pz.dev<double>();
   CK(allow_smem((const void*)k_fft_rows<double, kNtC>));
   CK(allow_smem((const void*)k_fft_cols<double, kNtC>));
@@ -1079,8 +1093,7 @@ void build_dmatrix(dda_ctx* c) {
                                             c->px.pos, c->py.pos, c->pz.pos);
     CK(cudaGetLastError());
   }
-  CK(cudaFreeAsync(full, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  CK(cudaFreeAsync(full, c->stream));  // (a synchronisation would give the block back to the driver)
 }
 
 // Host-supplied D (reference layout, reference units) -> octants.
