@@ -64,20 +64,20 @@ def parse():
     return ap.parse_args()
 
 
-# DRAM traffic per launch of the y/z plane kernel (dram__bytes_read.sum +
-# dram__bytes_write.sum), from ncu captures of `bench.py --matvec-only`:
-#   box:       the default workload, FP32, 2 rhs (captured at full size; the
-#              planes stay in L2, so the DRAM bytes are the first reads only)
-#   spheroid:  the 128-rhs block's kernel captured at 8 rhs; the traffic is
-#              a fixed part (D octant, tables) plus a part per rhs, so a full
-#              launch is fixed + 128 * per_rhs
-# Summaries with the commands: profiles/k_yz_p_box10x5x5_fp32.md,
-# profiles/k_yz_p_spheroid_fp32.md.
-TRAFFIC = {"box": {"fixed": 36663637, "per_rhs": 0, "rhs": 2},      # L2-resident planes: reads only
-           "spheroid": {"fixed": 14340480, "per_rhs": 39347072}}
+# DRAM traffic of one matvec's y/z passes (dram__bytes_read.sum +
+# dram__bytes_write.sum of k_zfwd, k_rows and k_zinv, L2 as the launch before
+# left it), from ncu captures of `bench.py --matvec-only`:
+#   box:       the default workload, FP32, 2 rhs (the work buffer stays in L2 in
+#              part)
+#   spheroid:  the 128-rhs block's kernels captured at 8 and 16 rhs: a fixed part
+#              (D octant, tables) and a part per rhs
+# Summaries with the commands: profiles/yz_passes_box10x5x5_fp32.md,
+# profiles/yz_passes_spheroid_fp32.md.
+TRAFFIC = {"box": {"fixed": 75313408, "per_rhs": 0, "rhs": 2},
+           "spheroid": {"fixed": 23286272, "per_rhs": 197693056}}
 
 
-def traffic_per_launch(workload, nrhs):
+def yz_traffic(workload, nrhs):
     t = TRAFFIC.get(workload)
     if t is None or ("rhs" in t and t["rhs"] != nrhs):
         return None
@@ -278,18 +278,22 @@ def build_problem(precision, max_rhs):
     return p, mv, np.concatenate(ein)
 
 
+def stage_names(mv):
+    """The stages of a matvec: x forward, y/z (three kernels or a plane
+    kernel), x inverse."""
+    return ["x_forward", "yz_passes" if mv.passes else "yz_plane_kernel", "x_inverse"]
+
+
 def stage_bytes(p, mv, nrhs, s):
-    """Algorithmic bytes per launch of the three matvec passes."""
+    """Algorithmic bytes per matvec of its three stages."""
     gx, gy, gz = p.grid
     bx, by, bz = p.box
     nvs, nv = p.nvs, p.nv
     plane = gx * by * bz
     oct_ = (gx // 2 + 1) * (gy // 2 + 1) * (gz // 2 + 1)
-    return {
-        "x_forward": nrhs * s * (3 * nvs + 3 * plane) + 13 * nv,
-        "yz_planes": nrhs * s * 6 * plane + s * 6 * oct_,
-        "x_inverse": nrhs * s * (6 * nvs + 3 * plane) + 13 * nv,
-    }
+    return dict(zip(stage_names(mv), (nrhs * s * (3 * nvs + 3 * plane) + 13 * nv,
+                                      nrhs * s * 6 * plane + s * 6 * oct_,
+                                      nrhs * s * (6 * nvs + 3 * plane) + 13 * nv)))
 
 
 def run_ours(args):
@@ -373,10 +377,10 @@ def run_ours(args):
            "h2d_bytes_per_step": int(einc_host.nbytes), "d2h_bytes_per_step": int(einc_host.nbytes),
            "host_arrays": "complex64 (dda_solve_f32)" if prec == "fp32" else "complex128 (dda_solve)"}
 
-    # matvec stage profile and roofline of the dominant pass
+    # matvec stage profile and roofline of the dominant stage
     ms = mv.profile(nrhs=nrhs, reps=20)
     sb = stage_bytes(p, mv, nrhs, s_bytes)
-    names = ["x_forward", "yz_planes", "x_inverse"]
+    names = stage_names(mv)
     dom = int(np.argmax(ms[:3]))
     peaks = {}
     try:
@@ -387,9 +391,9 @@ def run_ours(args):
     achieved = sb[names[dom]] / (ms[dom] * 1e-3) / 1e9
     roofline = {"bound": "hbm", "kernel": names[dom], "achieved": achieved, "peak": peak,
                 "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic_per_launch("box", nrhs) if (prec == "fp32" and names[dom] == "yz_planes") else None,
+                "traffic": yz_traffic("box", nrhs) if (prec == "fp32" and names[dom] == "yz_passes") else None,
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
-                "algorithmic_bytes_per_launch": sb[names[dom]], "ms_per_launch": float(ms[dom])}
+                "algorithmic_bytes_per_matvec": sb[names[dom]], "ms_per_matvec": float(ms[dom])}
     matvec = {"ms": float(ms[3]), "stages_ms": dict(zip(names, map(float, ms[:3]))),
               "GB_per_s": sum(sb.values()) / (ms[3] * 1e-3) / 1e9, "nrhs": nrhs}
 

@@ -46,7 +46,7 @@ def _peaks():
 def _roofline(p, mv, nrhs, s_bytes, reps=5):
     ms = mv.profile(nrhs=nrhs, reps=reps)
     sb = bench.stage_bytes(p, mv, nrhs, s_bytes)
-    names = ["x_forward", "yz_planes", "x_inverse"]
+    names = bench.stage_names(mv)
     dom = int(np.argmax(ms[:3]))
     peaks = _peaks()
     peak = float(peaks.get("hbm_gbs", 6650.0))
@@ -55,7 +55,7 @@ def _roofline(p, mv, nrhs, s_bytes, reps=5):
     return ({"bound": "hbm", "kernel": names[dom], "achieved": achieved, "peak": peak, "unit": "GB/s",
              "frac": achieved / peak, "traffic": None,
              "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
-             "algorithmic_bytes_per_launch": sb[names[dom]], "ms_per_launch": float(ms[dom])},
+             "algorithmic_bytes_per_matvec": sb[names[dom]], "ms_per_matvec": float(ms[dom])},
             {"ms": float(ms[3]), "stages_ms": dict(zip(names, map(float, ms[:3]))),
              "GB_per_s": total / (ms[3] * 1e-3) / 1e9, "frac_of_hbm": total / (ms[3] * 1e-3) / 1e9 / peak,
              "nrhs": nrhs, "algorithmic_bytes": total})
@@ -182,7 +182,7 @@ def batched_block(steps, warmup, local=0, nrhs=128, cpu=True):
     e2e = {"value": nrhs * n_e2e / (e2e_ms / 1000.0), "unit": "solves/s",
            "h2d_bytes_per_step": int(einc.nbytes), "d2h_bytes_per_step": int(einc.nbytes)}
     roof, matvec = _roofline(p, mv, nrhs, 8, reps=3)
-    roof["traffic"] = bench.traffic_per_launch("spheroid", nrhs)
+    roof["traffic"] = bench.yz_traffic("spheroid", nrhs)
     layout = mv.layout
     mv.close()
     del e_dev, pol_dev, einc_host, pol_host

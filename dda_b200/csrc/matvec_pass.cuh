@@ -8,8 +8,10 @@
 //
 // k_yz_p keeps a whole plane in one CTA's shared memory, so an SM holds one
 // CTA of 16 warps whose stages all end at its barriers.  Here a CTA holds a
-// column tile or a few rows (8 to 40 KB), an SM holds several CTAs in
-// different phases, and every global access is the first or last butterfly
+// column tile (256 bytes of every kz: 2 KB at Gz = 8, 64 KB at 256; half of that
+// beyond) or a few rows (up to 48 KB, see RTile), with the twiddles and in the
+// row kernel a D-hat row beside them; an SM holds several CTAs in different
+// phases, and every global access is the first or last butterfly
 // stage of a line: inputs go from HBM or L2 to registers, outputs from
 // registers back, and each transform passes through shared memory K - 1
 // times for a K-stage plan.
@@ -21,11 +23,11 @@
 //
 // What bounds them and what they take (16 right-hand sides of the spheroid,
 // planes 128 x 128 with by = bz = 64, FP32, W = 2; HBM floor at 6.5 TB/s): z
-// forward 148 us and z inverse 156 us of 140 us (HBM); rows 383 us of 188 us,
-// of which the FMA pipe is busy 205 us and the shared-memory pipe 215 us, with
-// 14 warps an SM (128 registers) the latency between the two.  The plane
-// kernel took 1 202 us for all of it; 128 right-hand sides 9.41 -> 5.39 ms,
-// 512^3 (two) 12.9 -> 5.9 ms (cluster kernel).  W = 1 instead of 2: rows 424
+// forward 148 us and z inverse 154 us of 140 us (HBM); rows 395 us of 188 us,
+// with the FMA pipe busy 56 % of the time, the shared-memory pipe 65 %, and
+// 13 warps an SM (128 registers) to cover the latency between the two.  The
+// plane kernel took 1 202 us for all of it; 128 right-hand sides 9.41 -> 5.39 ms,
+// 512^3 (two) 12.9 -> 6.5 ms (cluster kernel).  W = 1 instead of 2: rows 424
 // us.  Twiddles from global memory through L1 instead of shared memory: rows
 // 492 us, z forward 182 us.
 //
@@ -201,7 +203,9 @@ template <typename V, typename P> struct ZTile {
 // four rows 79.5 us, two 90.4; 512: one row 974 us, four 2 400).  Registers per
 // thread: as many as leave the most warps without spills that cost more (FP64,
 // 16 x 8: 128 registers 482 us, 160 438; 20 x 5: 89 and 95; P2, 16 x 8: 383 and
-// 407; FP32, 32 x 8: 80 registers 296 us, 96 286).
+// 407; FP32, 32 x 8: 80 registers 296 us, 96 286).  Measured at these plans;
+// others take the limit of the nearest, and in FP64 30 x 6 and 30 x 7 spill 152
+// bytes at 128, as k_zfwd does 112 to 160 with first radices of 30 and 32.
 template <typename V, typename P> struct RTile {
   enum : int {
     LINE = 3 * RowPad<P>::pitch(sizeof(V)) * (int)sizeof(V),
