@@ -72,22 +72,23 @@ typedef struct dda_problem {
   uint32_t flags;            /* DDA_FLAG_* */
 } dda_problem;
 
-/* dda_problem.flags: run the y/z passes through three kernels and a plane
- * buffer even when a kx plane fits in shared memory (the path large grids
- * take); used by tests and tuning. */
+/* dda_problem.flags: run the y/z part through column FFTs along z and a row
+ * kernel over a buffer of whole planes (the path of runtime-planned grids whose
+ * kx plane fits neither a CTA nor a cluster); used by tests and tuning. */
 #define DDA_FLAG_SPLIT_YZ 1u
 /* dda_problem.flags: use the runtime-planned FFT kernels even when every grid
  * edge has a compile-time plan; used by tests and tuning. */
 #define DDA_FLAG_RUNTIME_PLANS 2u
 /* dda_problem.flags: run the y/z passes through the cluster kernel (a
  * thread-block cluster per kx plane exchanging through an L2-resident plane
- * buffer, the path for planes beyond one CTA's shared memory) even when a
- * plane fits; used by tests and tuning.  DDA_FLAG_SPLIT_YZ takes precedence. */
+ * buffer, the path of runtime-planned grids whose planes are beyond one CTA's
+ * shared memory) on any grid; used by tests and tuning.  DDA_FLAG_SPLIT_YZ takes precedence. */
 #define DDA_FLAG_SLOT_YZ 4u
 /* dda_problem.flags: keep the default y/z batching instead of timing the
  * candidates at dda_create (the autotuner picks, per grid shape, the rows
  * per batch of the plane kernels and the cluster size of the cluster
- * kernel; neither changes the results). */
+ * kernel; neither changes the results; grids of the y/z passes have nothing
+ * to tune). */
 #define DDA_FLAG_NO_AUTOTUNE 8u
 /* dda_problem.flags: launch every solver iteration kernel by kernel instead of
  * replaying captured CUDA graphs of two iterations (the results are the
@@ -95,14 +96,14 @@ typedef struct dda_problem {
 #define DDA_FLAG_NO_GRAPHS 16u
 /* dda_problem.flags: run the fused plane kernel as two groups of half the
  * CTA (or, with DDA_FLAG_YZ_GROUPS4, four groups of a quarter) with their own
- * barriers (the autotuner otherwise chooses between one, two and four
- * groups; the results are the same); used by tests. */
+ * barriers, also on grids that otherwise run the y/z passes (where those do
+ * not, the autotuner otherwise chooses between one, two and four groups; the
+ * results are the same); used by tests. */
 #define DDA_FLAG_YZ_GROUPS2 32u
 #define DDA_FLAG_YZ_GROUPS4 64u
 /* dda_problem.flags: run the planned y/z passes with one kx plane per cluster
- * of two CTAs (each holding half the plane; the autotuner otherwise chooses
- * between this and one CTA per plane; the results are the same); used by
- * tests. */
+ * of two CTAs (each holding half the plane), also on grids that otherwise run
+ * the three kernels of the passes (the results are the same); used by tests. */
 #define DDA_FLAG_YZ_PAIR 128u
 /* dda_problem.flags: keep the work buffer of the y/z passes (by default up to
  * 1 GiB per precision, which is fastest) within the memory that dda_create
@@ -214,8 +215,9 @@ int64_t dda_launch_count(const dda_ctx* ctx);
 
 /* FFT grid for a particle box.  DDA_GRID_REFERENCE: fftFit(2 box) per axis,
  * the reference's choice (DDA/DDAParams.cpp:290-335).  DDA_GRID_TUNED: per
- * axis the smallest length >= 2 box with compile-time FFT plans, y and z
- * equal so the y/z passes use them, unless that more than doubles the grid.
+ * axis the smallest of the 22 lengths >= 2 box that the plane kernels are tuned
+ * for, y and z equal, unless that more than doubles the grid (every even
+ * 2,3,5,7-smooth length up to 512 has compile-time FFT plans).
  * Any grid >= 2 box gives the same matvec up to rounding (the zero padding
  * makes the circular convolution the exact linear one); the reference's
  * --fft-grid sets it the same way. */

@@ -63,7 +63,8 @@ typedef struct dda_serve_result {
   double cext[2], cabs[2];   /* cross sections, m^2 (DDA/Beam.cpp:126-133, DDA/AbsCross.cpp:28-48) */
   double t_submit, t_admit, t_done;  /* seconds on the server clock */
   double t_setup, t_solved;  /* context built (D matrix included); solve finished */
-  int64_t footprint;         /* bytes reserved at admission (dda_footprint peak) */
+  int64_t footprint;         /* bytes reserved at admission (dda_footprint peak, with
+                                DDA_FLAG_SMALL_WORK where the budget had no room for more) */
   int64_t device_bytes;      /* bytes the request's context held */
   uint32_t grid[3];
   uint32_t nv;
@@ -79,7 +80,8 @@ typedef struct dda_serve_result {
 int dda_serve_create(int device, int64_t hbm_budget, int max_active, dda_server** out);
 
 /* Queues a request (its arrays are copied; the call does not wait for the
- * GPU).  Rejects a request whose footprint exceeds the whole budget. */
+ * GPU).  Rejects a request whose footprint with DDA_FLAG_SMALL_WORK exceeds the
+ * whole budget. */
 int dda_serve_submit(dda_server* s, const dda_serve_request* req, int64_t* id);
 
 /* Moves up to `max` finished results to `out`, waiting up to timeout_ms
